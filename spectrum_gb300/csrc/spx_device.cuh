@@ -185,8 +185,15 @@ __device__ __forceinline__ uint4 rng_block(uint64_t seed, uint32_t index, uint32
                         make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
 }
 
-// u = (x + 1/2) 2^-32 in (0,1)
-__device__ __forceinline__ double u01d(uint32_t x) { return ((double)x + 0.5) * 2.3283064365386962890625e-10; }
+// u = (x + 1/2) 2^-32 in (0,1). Double: (2x + 1) 2^-33 is exact, so its bits are put together by integer
+// operations (a conversion, an addition and a multiplication would each hold the FP64 pipe for 64 cycles of
+// the warp's scheduler).
+__device__ __forceinline__ double u01d(uint32_t x)
+{
+   const unsigned long long m = 2ull * x + 1ull;
+   const int e = 63 - __clzll((long long)m);
+   return __longlong_as_double((long long)(((unsigned long long)(1023 - 33 + e) << 52) + ((m << (52 - e)) - (1ull << 52))));
+}
 __device__ __forceinline__ float u01f(uint32_t x) { return __fmaf_rn((float)x, 2.3283064365386962890625e-10f, 1.16415321826934814453125e-10f); }
 template <class R> __device__ __forceinline__ R u01(uint32_t x);
 template <> __device__ __forceinline__ double u01<double>(uint32_t x) { return u01d(x); }

@@ -1,0 +1,52 @@
+"""The step's special paths against the general ones: what a path takes over gives the same trajectories.
+
+- Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
+  and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
+  kernels of one diffusion class against the kernel that dispatches at run time, whose steps are general."""
+import numpy as np
+import pytest
+
+import oracle_tools as ot
+import test_oracle_plugins as cases
+from spectrum_gb300 import capi
+from spectrum_gb300.datacontainer import DataContainer as DC
+from spectrum_gb300.plugins import DiffusionRigidityMagneticFieldPowerLaw
+from spectrum_gb300.simulation import open_problems, run_problems
+
+pytestmark = pytest.mark.gpu
+
+UNIFORM_DIFFUSION = {
+    "full": (cases.DiffusionFullConstant(), DC().double(0.5).double(2.0)),
+    "rigidity_b": (DiffusionRigidityMagneticFieldPowerLaw(),
+                   DC().double(0.3).double(5.0).double(0.7).double(0.5).double(1.0).double(0.1)),
+    "radial": cases.DIFFUSION_CASES["kin_energy_radial"][0],  # reads the position: the general step
+}
+
+
+def _uniform(name, flow, n):
+    bg = (cases.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((0.2, 0.1, -0.1)).vec((0.3, -0.2, 0.8)).double(0.05))
+    return cases._parker(n=n, bg=bg, diff=UNIFORM_DIFFUSION[name], flow=flow, t_end=0.1 if flow == cases.FORWARD else -0.1,
+                         is_=(cases.InitialSpaceFixed(), DC().vec((0.3, 0, 0))),
+                         bnds=[(cases.BoundarySphereReflect(), cases.B(DC(), -1, [-1]).vec((0, 0, 0)).double(0.6))])
+
+
+@pytest.mark.parametrize("flow", [cases.FORWARD, cases.BACKWARD])
+@pytest.mark.parametrize("name", sorted(UNIFORM_DIFFUSION))
+def test_uniform_field_matches_oracle(built_lib, name, flow):
+    pb = _uniform(name, flow, 33)
+    res = run_problems(pb, precision=capi.SPX_FP64, record=True)
+    ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
+
+
+@pytest.mark.parametrize("flow", [cases.FORWARD, cases.BACKWARD])
+@pytest.mark.parametrize("name", ["full", "rigidity_b"])
+def test_uniform_field_fp32_equals_the_general_step(built_lib, name, flow):
+    rec = []
+    for special in (0, 1):
+        sim = open_problems(_uniform(name, flow, 1000), precision=capi.SPX_MIXED, record=True)
+        sim.ctx.set_option(capi.SPX_OPT_SPECIALIZE, float(special))
+        sim.MainLoop()
+        rec.append(sim.ctx.records(0, 1000))
+        sim.close()
+    for f in ("status", "steps", "t", "pos", "mom"):
+        assert np.array_equal(rec[0][f], rec[1][f]), f
