@@ -16,13 +16,20 @@ template <> struct Units<float> {
    static constexpr float c = (float)(2.99792458e+10 / (0.1 * 2.99792458e+10));
 };
 template <class R> __device__ __forceinline__ R c_code() { return Units<R>::c; }
+// x / c and x / (2 c)
+__device__ __forceinline__ double over_c(double x) { return Divisor<double>(Units<double>::c, 1.0 / Units<double>::c)(x); }
+__device__ __forceinline__ float over_c(float x) { return x / Units<float>::c; }
+__device__ __forceinline__ double over_2c(double x) { return Divisor<double>(2.0 * Units<double>::c, 1.0 / (2.0 * Units<double>::c))(x); }
+__device__ __forceinline__ float over_2c(float x) { return x / (2.0f * Units<float>::c); }
+template <class R> __device__ __forceinline__ V3<R> over_c(V3<R> a) { return {over_c(a.x), over_c(a.y), over_c(a.z)}; }
+template <class R> __device__ __forceinline__ V3<R> over_2c(V3<R> a) { return {over_2c(a.x), over_2c(a.y), over_2c(a.z)}; }
 template <class R> __device__ __forceinline__ R enr_tot(R p) { R c = c_code<R>(); return m_sqrt(p * p + c * c) * c; }
 template <class R> __device__ __forceinline__ R enr_kin(R p) { R c = c_code<R>(); return enr_tot(p) - c * c; }
 template <class R> __device__ __forceinline__ R vel_of(R p) { R c = c_code<R>(); return p * (c * c) / enr_tot(p); }
 template <class R> __device__ __forceinline__ R mom_of(R e) { R c = c_code<R>(); return m_sqrt(e * (e + R(2) * (c * c))) / c; }
 template <class R> __device__ __forceinline__ R rigidity(R p) { return p * c_code<R>(); }
-template <class R> __device__ __forceinline__ R larmor(R p, R b) { return p * c_code<R>() / b; }
-template <class R> __device__ __forceinline__ R rel_factor(R v) { R r = v / c_code<R>(); return R(1) / m_sqrt(R(1) - r * r); }
+template <class R> __device__ __forceinline__ R larmor(R p, R b) { return quot(p * c_code<R>(), b); }
+template <class R> __device__ __forceinline__ R rel_factor(R v) { R r = over_c(v); return R(1) / m_sqrt(R(1) - r * r); }
 template <class R> __device__ __forceinline__ R cyclotron(R v, R b) { return b / (rel_factor(v) * c_code<R>()); }
 template <class R> __device__ __forceinline__ V3<R> vel_cart(V3<R> mom) { R m = norm(mom); return (vel_of(m) / m) * mom; }
 
@@ -51,7 +58,7 @@ template <class R> __device__ __forceinline__ V3<R> sd_b_gradbhat(const SD<R>& s
 // div U, divbhat and bhat.grad(bhat) from the gradient matrices (common/spatial_data.hh:213-330)
 template <class R> __device__ __forceinline__ R mat_divbhat(const SD<R>& s)
 {
-   return (trace(s.gradB) - dot(s.gradBmag, s.bhat)) / s.Bmag;
+   return quot(trace(s.gradB) - dot(s.gradBmag, s.bhat), s.Bmag);
 }
 template <class R> __device__ __forceinline__ V3<R> mat_b_gradbhat(const SD<R>& s)
 {
@@ -61,7 +68,7 @@ template <class R> __device__ __forceinline__ V3<R> mat_b_gradbhat(const SD<R>& 
    for (int j = 0; j < 3; j++) {
       R acc = R(0);
 #pragma unroll
-      for (int i = 0; i < 3; i++) acc += s.bhat[i] * ((s.gradB.m[i][j] - s.gradBmag[i] * s.bhat[j]) / s.Bmag);
+      for (int i = 0; i < 3; i++) acc += s.bhat[i] * quot(s.gradB.m[i][j] - s.gradBmag[i] * s.bhat[j], s.Bmag);
       o[j] = acc;
    }
    r = {o[0], o[1], o[2]};
@@ -135,7 +142,7 @@ __device__ __forceinline__ void eval_bg(const BgParamsT<R>& g, R t, V3<R> pos, u
       R a1 = shock_tr(g.tanh_k, ds), a2 = R(1) - a1;
       if ((mask & kU) || (mask & kE)) s.U = a1 * ld3(g.u0) + a2 * ld3(g.u1);
       if (mask & kB) s.B = a1 * ld3(g.B0) + a2 * ld3(g.B1);
-      if (mask & kE) s.E = R(-1) * (cross(s.U, s.B) / c_code<R>());  // InducedEfield: -(U x B) / c
+      if (mask & kE) s.E = R(-1) * over_c(cross(s.U, s.B));  // InducedEfield: -(U x B) / c
       R rg = R(1) * a1 + R(2) * a2;
       s.region = mk(rg, rg, rg);
    }
@@ -154,7 +161,7 @@ __device__ __forceinline__ void eval_bg(const BgParamsT<R>& g, R t, V3<R> pos, u
    }
    else if (BG == kBgSolarWind) {  // src/background_solarwind.cc:111-255, switches at their defaults
       V3<R> pp = eframe_to(g, pos - ld3(g.r0));
-      R r = norm(pp), r_mns = r - g.r_ref, costheta = pp.z / r, ur = g.ur0;
+      R r = norm(pp), r_mns = r - g.r_ref, costheta = quot(pp.z, r), ur = g.ur0;
       s.region = mk(r < R(117.0 * 1.495978707E+13 / 1.0e10) ? R(1) : R(-1), R(-1), s.region.z);
       // U also when only E is asked for (the Lorentz mask): E = -U x B / c needs it (deviation D4)
       if (mask & (kU | kE)) s.U = eframe_from(g, ur * unit(pp));
@@ -162,13 +169,13 @@ __device__ __forceinline__ void eval_bg(const BgParamsT<R>& g, R t, V3<R> pos, u
          R sintheta = m_sqrt(m_max(R(1) - costheta * costheta, R(0)));
          R sr = m_sqrt(pp.x * pp.x + pp.y * pp.y), cosphi, sinphi;
          if (sr < r * Lim<R>::tiny) { cosphi = R(0); sinphi = R(0); }
-         else { cosphi = pp.x / sr; sinphi = pp.y / sr; }
-         R q = g.r_ref / r;
+         else { const Divisor<R> d(sr); cosphi = d(pp.x); sinphi = d(pp.y); }
+         R q = quot(g.r_ref, r);
          R Br = g.B0[0] * (q * q);
          R Bp = -Br * sintheta * r_mns * g.w0 / ur;
          s.B = eframe_from(g, mk(Br * sintheta * cosphi - Bp * sinphi, Br * sintheta * sinphi + Bp * cosphi, Br * costheta));
       }
-      if (mask & kE) s.E = R(-1) * (cross(s.U, s.B) / c_code<R>());  // InducedEfield: -(U x B) / c
+      if (mask & kE) s.E = R(-1) * over_c(cross(s.U, s.B));  // InducedEfield: -(U x B) / c
    }
    else if (BG == kBgGrid) grid_reader_values(g, pos, s);  // the points of numerical derivatives (order -1)
 }
@@ -209,7 +216,7 @@ __device__ __forceinline__ bool solarwind_closed(const BgParamsT<R>& g, V3<R> po
    V3<R> w = cross(x, O);
    s.U = (g.ur0 * ir) * x;
    s.B = (g.A * ir3) * x + (k * f) * w;
-   if (mask & kE) s.E = R(-1) * (cross(s.U, s.B) / c_code<R>());  // InducedEfield: -(U x B) / c
+   if (mask & kE) s.E = R(-1) * over_c(cross(s.U, s.B));  // InducedEfield: -(U x B) / c
    s.Bmag = norm(s.B);
    if (!(s.Bmag >= Lim<R>::tiny)) return false;
    R iB = R(1) / s.Bmag;
@@ -543,10 +550,10 @@ __device__ __noinline__ void numerical_derivs(const BgParamsT<R>& g, R t, V3<R> 
          dr *= R(2);
          pt = pt - dr * fa[xyz];
          eval_bg<BG>(g, t, pt, m1, b, ds);
-         if (m1 & kU) { gu.m[xyz][0] = (f.U.x - b.U.x) / dr; gu.m[xyz][1] = (f.U.y - b.U.y) / dr; gu.m[xyz][2] = (f.U.z - b.U.z) / dr; }
+         if (m1 & kU) { gu.m[xyz][0] = quot(f.U.x - b.U.x, dr); gu.m[xyz][1] = quot(f.U.y - b.U.y, dr); gu.m[xyz][2] = quot(f.U.z - b.U.z, dr); }
          if (m1 & kB) {
-            gbv.m[xyz][0] = (f.B.x - b.B.x) / dr; gbv.m[xyz][1] = (f.B.y - b.B.y) / dr; gbv.m[xyz][2] = (f.B.z - b.B.z) / dr;
-            gbm[xyz] = (norm(f.B) - norm(b.B)) / dr;
+            gbv.m[xyz][0] = quot(f.B.x - b.B.x, dr); gbv.m[xyz][1] = quot(f.B.y - b.B.y, dr); gbv.m[xyz][2] = quot(f.B.z - b.B.z, dr);
+            gbm[xyz] = quot(norm(f.B) - norm(b.B), dr);
          }
          s.dr[xyz] = dr;
       }
@@ -644,7 +651,7 @@ __device__ __forceinline__ bool get_fields(const BgParamsT<R>& g, int deriv_mode
       for (int a = 0; a < 3; a++)
 #pragma unroll
          for (int b = 0; b < 3; b++)
-            s.gradB.m[a][b] = R(3) * (M[a] * pp[b] + pp[a] * M[b] + mr * ((a == b ? R(1) : R(0)) - R(5) * (pp[a] * pp[b]) / r2)) / r5;
+            s.gradB.m[a][b] = quot(R(3) * (M[a] * pp[b] + pp[a] * M[b] + mr * ((a == b ? R(1) : R(0)) - quot(R(5) * (pp[a] * pp[b]), r2))), r5);
       s.gradBmag = mv(s.gradB, s.bhat);
       s.dUdt = mk(R(0), R(0), R(0));
    }

@@ -564,15 +564,14 @@ __device__ __forceinline__ bool space_terminate(Lane<R, A>& L, BndView<R> bv, co
 template <class R>
 __device__ __forceinline__ R time_proximity(R dt, R dmax, BndView<R> bv, int nbt, bool fwd)
 {
-   R c = c_code<R>();
-   R dn = fwd ? -Lim<R>::large * dmax / c : Lim<R>::large * dmax / c;
+   R dn = over_c(fwd ? -Lim<R>::large * dmax : Lim<R>::large * dmax);
    for (int b = 0; b < nbt; b++) {
       R delta = bv.ld(b).delta;
       if (fwd) { if (delta <= R(0) && delta > dn) dn = delta; }
       else { if (delta >= R(0) && delta < dn) dn = delta; }
    }
-   if (fwd) { if (dt >= -dn) dt = m_max(-(R(1) + Lim<R>::little) * dn, Lim<R>::small * dmax / c); }
-   else { if (dt >= dn) dt = m_max((R(1) + Lim<R>::little) * dn, Lim<R>::small * dmax / c); }
+   if (fwd) { if (dt >= -dn) dt = m_max(-(R(1) + Lim<R>::little) * dn, over_c(Lim<R>::small * dmax)); }
+   else { if (dt >= dn) dt = m_max((R(1) + Lim<R>::little) * dn, over_c(Lim<R>::small * dmax)); }
    return dt;
 }
 
@@ -599,7 +598,7 @@ __device__ __forceinline__ void track_bmag(Start& s0, const RunConfig& cfg, cons
 template <class R, class A>
 __device__ __forceinline__ bool prev_step_ok(Lane<R, A>& L, R dmax)
 {
-   if (L.steps > 0 && !(L.dt >= Lim<R>::tiny * dmax / c_code<R>())) {
+   if (L.steps > 0 && !(L.dt >= over_c(Lim<R>::tiny * dmax))) {
       L.status |= TRAJ_DISCARD;
       return false;
    }
@@ -627,7 +626,7 @@ __device__ __noinline__ bool parker_divk_fd(const ProblemDescT<R>& P, int deriv_
       for (int i = 0; i < 3; i++) {
          R f = kf.perp * (i == j ? R(1) : R(0)) + (kf.para - kf.perp) * sf.bhat[j] * sf.bhat[i];
          R b = kb.perp * (i == j ? R(1) : R(0)) + (kb.para - kb.perp) * sb.bhat[j] * sb.bhat[i];
-         dk[i] += R(0.5) * (f - b) / delta;
+         dk[i] += quot(R(0.5) * (f - b), delta);
       }
    }
    divK = mk(dk[0], dk[1], dk[2]);
@@ -1071,15 +1070,14 @@ __device__ __forceinline__ V3<R> guiding_drift(const SD<R>& s, V3<R> mom, V3<R> 
 {
    const R c = c_code<R>();
    const R rL = larmor(mom.x, s.Bmag), rR = larmor(mom.z, s.Bmag);
-   const V3<R> zero3 = mk(R(0), R(0), R(0));
-   V3<R> dbhatdt = (zero3 - R(0) * s.bhat) / s.Bmag;
    V3<R> curlbhat = (sd_curlB(s) - cross(s.gradBmag, s.bhat)) / s.Bmag;
-   V3<R> e_star = (s.E - ((rR * s.Bmag) * dbhatdt) / c) - ((rL * vel.x) * s.gradBmag) / (R(2) * c);
+   // d bhat / dt is zero in the static backgrounds of this family, and with it E's term in it
+   V3<R> e_star = s.E - over_2c((rL * vel.x) * s.gradBmag);
    V3<R> b_star = s.B + (rR * s.Bmag) * curlbhat;
    R bsb = dot(b_star, s.bhat);
    V3<R> drift = (vel.z * b_star + c * cross(e_star, s.bhat)) / bsb;
-   dp_perp = R(0.5) * mom.x / s.Bmag * (R(0) + dot(drift, s.gradBmag));
-   dp_para = dot(e_star, b_star) / bsb;  // the proton's charge is 1 in code units
+   dp_perp = quot(R(0.5) * mom.x, s.Bmag) * (R(0) + dot(drift, s.gradBmag));
+   dp_para = quot(dot(e_star, b_star), bsb);  // the proton's charge is 1 in code units
    return drift;
 }
 
@@ -1136,7 +1134,7 @@ __device__ __forceinline__ void rk_slopes(const SD<R>& s, V3<R> mom, V3<R> vel, 
 {
    if (TT == kLorentz) {  // src/trajectory_lorentz.cc:67-71
       sp = vel;
-      sm = s.E + cross(vel, s.B) / c_code<R>();
+      sm = s.E + over_c(cross(vel, s.B));
    }
    else if (TT == kFieldline) {  // src/trajectory_fieldline.cc:58-66: along b at the parallel speed
       sp = vel.z * s.bhat;

@@ -1,5 +1,7 @@
 """The step's special paths against the general ones: what a path takes over gives the same trajectories.
 
+- Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
+  1e140 takes the time-step bounds there (FP64 against the oracle).
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
   and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
   kernels of one diffusion class against the kernel that dispatches at run time, whose steps are general."""
@@ -50,3 +52,10 @@ def test_uniform_field_fp32_equals_the_general_step(built_lib, name, flow):
         sim.close()
     for f in ("status", "steps", "t", "pos", "mom"):
         assert np.array_equal(rec[0][f], rec[1][f]), f
+
+
+def test_quotients_outside_the_fast_range(built_lib):
+    bg = (cases.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((0, 0, 0)).vec((0, 0, 1.0)).double(1.0e140))
+    pb = cases._parker(n=40, bg=bg, t_end=0.1)
+    res = run_problems(pb, precision=capi.SPX_FP64, record=True)
+    ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
