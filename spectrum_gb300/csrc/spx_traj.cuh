@@ -903,10 +903,6 @@ struct FixedRk {
    static constexpr bool kGeneral = false;
    __host__ __device__ static constexpr int stages() { return S; }
    template <class R> __device__ __forceinline__ R a(int s) const { return s == 0 ? R(0) : (s == 3 ? R(1) : R(0.5)); }
-   template <class R> __device__ __forceinline__ R b(int s, int l) const
-   {
-      return (s == 1 && l == 0) ? R(0.5) : ((s == 2 && l == 1) ? R(0.5) : ((s == 3 && l == 2) ? R(1) : R(0)));
-   }
    template <class R> __device__ __forceinline__ R v(int l) const
    {
       return S == 1 ? R(1) : ((l == 0 || l == 3) ? R(1.0 / 6.0) : R(1.0 / 3.0));
@@ -1424,12 +1420,24 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
    }
    // RKSlopes: stage "is" (false: the trajectory ended or was discarded in it)
    auto stage = [&](int is) -> bool {
+      if constexpr (TAB::kGeneral) {
 #pragma unroll
-      for (int il = 0; il < is; il++) {
-         R ds = L.dt * tab.template b<R>(is, il);
-         R dta = tab.template a<R>(is) * L.dt;
-         if (fwd) { acc_add(L.t, dta); add3(L.pos, ds * slp[il]); add3(L.mom, ds * slm[il]); }
-         else { acc_add(L.t, -dta); add3(L.pos, R(-1) * (ds * slp[il])); add3(L.mom, R(-1) * (ds * slm[il])); }
+         for (int il = 0; il < is; il++) {
+            R ds = L.dt * tab.template b<R>(is, il);
+            R dta = tab.template a<R>(is) * L.dt;
+            if (fwd) { acc_add(L.t, dta); add3(L.pos, ds * slp[il]); add3(L.mom, ds * slm[il]); }
+            else { acc_add(L.t, -dta); add3(L.pos, R(-1) * (ds * slp[il])); add3(L.mom, R(-1) * (ds * slm[il])); }
+         }
+      }
+      else {
+         // the fixed tables have one nonzero coefficient a stage, that of the stage before; the reference
+         // advances t once for every earlier stage. (Adding the zero products cost ten float operations each:
+         // the FP32 dipole orbits take 42.4 ms instead of 51.0, guiding centres 38.4 instead of 43.6.)
+         const R dta = tab.template a<R>(is) * L.dt, ds = fwd ? dta : -dta;
+#pragma unroll
+         for (int il = 0; il < is; il++) acc_add(L.t, ds);
+         add3(L.pos, ds * slp[is - 1]);
+         add3(L.mom, ds * slm[is - 1]);
       }
       if (space_terminate<TT>(L, bv, sp, s0, P, Pd, S)) return false;
       V3<R> ms = lane_mom(L);
