@@ -470,6 +470,34 @@ int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, spx_tuning& 
    return SPX_OK;
 }
 
+// The plain grid of a run: how many lanes of a warp hold trajectories, and in FP64 how many lanes share one.
+// The FP64 pipe takes a warp instruction every 64 cycles of each scheduler, whatever its active lanes, so up to
+// one warp per scheduler is free: a launch that fits spreads over all schedulers (fewer trajectories a warp
+// diverge less), and where the kernel evaluates finite differences or pairs of normals its trajectories
+// get up to eight lanes each. Larger launches take one lane each and full warps; a caller's own launch shape
+// is kept as given.
+struct PlainShape {
+   int64_t grid;
+   int block, warp_lanes, team;
+};
+
+PlainShape plain_shape(const spx_ctx* c, int64_t total, int block, bool chosen_here)
+{
+   PlainShape s{0, block, 32, 1};
+   const int64_t warps = (int64_t)c->sm_count * 4;  // one per scheduler
+   if (chosen_here && c->precision == SPX_FP64 && total <= warps * 32) {
+      const bool parker = c->traj == SPX_TRAJ_PARKER || c->traj == SPX_TRAJ_PARKER_SOURCE;
+      const bool fd = c->deriv_mode == 0 && c->bg_kind == spx::kBgSolarWind;
+      if (parker || fd)
+         while (s.team < 8 && total * s.team * 2 <= warps * 32) s.team *= 2;
+      s.warp_lanes = s.team * (int)std::max<int64_t>(1, (total + warps - 1) / warps);
+      s.block = 32;
+   }
+   const int64_t per_block = (int64_t)(s.block / 32) * (s.warp_lanes / s.team);
+   s.grid = (total + per_block - 1) / per_block;
+   return s;
+}
+
 
 // What a captured graph depends on: launch shape, the run configuration apart from the run
 // index, and the device buffers. A different key means a new capture.
@@ -930,11 +958,13 @@ int spx_run(spx_ctx_t c, const spx_tuning* tuning)
    const int trc = resolve_tuning(c, tuning, slots, tu);
    if (trc != SPX_OK) return trc;
    spx::LaunchArgs a;
+   const PlainShape ps = plain_shape(c, c->total_traj, tu.block_size, tuning == nullptr && !c->has_tuned);
+   if (tu.schedule == 0) tu.block_size = ps.block;
    a.block = dim3(tu.block_size);
-   int64_t grid;
-   if (tu.schedule == 1) grid = (int64_t)c->sm_count * tu.blocks_per_sm;  // persistent: fill the GPU once
-   else grid = (c->total_traj + tu.block_size - 1) / tu.block_size;      // one thread per trajectory
+   int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm : ps.grid;  // persistent: fill the GPU once
    grid = std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff));
+   a.cfg.warp_lanes = ps.warp_lanes;
+   a.cfg.team = ps.team;
    a.grid = dim3((unsigned)grid);
    a.stream = c->stream;
    a.problems_r = c->d_pr;
@@ -1054,6 +1084,8 @@ int spx_autotune(spx_ctx_t c, int64_t sample_traj, spx_tuning* best)
       int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * occ : (first + tu.block_size - 1) / tu.block_size;
       spx::LaunchArgs a;
       a.block = dim3(tu.block_size);
+      a.cfg.warp_lanes = 32;
+      a.cfg.team = 1;
       a.grid = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff)));
       a.stream = c->stream;
       a.problems_r = b_pr.p;
@@ -1582,7 +1614,9 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    const int slots = bnd_slots(c);
    rc = resolve_tuning(c, tuning, slots, tu);
    if (rc != SPX_OK) return rc;
-   int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm : (total + tu.block_size - 1) / tu.block_size;
+   const PlainShape ps = plain_shape(c, total, tu.block_size, tuning == nullptr && !c->has_tuned);
+   if (tu.schedule == 0) tu.block_size = ps.block;
+   int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm : ps.grid;
    grid = std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff));
 
    // descriptors into the scratch, counters cleared
@@ -1601,6 +1635,8 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    spx::LaunchArgs a;
    a.block = dim3(tu.block_size);
    a.grid = dim3((unsigned)grid);
+   a.cfg.warp_lanes = ps.warp_lanes;
+   a.cfg.team = ps.team;
    a.stream = c->stream;
    a.problems_r = scratch + off_pr;
    a.problems_d = reinterpret_cast<const spx::ProblemDesc*>(scratch + off_pd);

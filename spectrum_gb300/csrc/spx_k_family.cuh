@@ -12,8 +12,8 @@ namespace spx {
 
 template <int TT, class R, int DM, bool GT, int DK = -1, int BL = kLayoutAny>
 struct FamilyTU {
-   // dynamic shared memory: the boundary states of every lane of a block
-   static size_t smem(int slots, int block) { return (size_t)(slots > 0 ? slots : 1) * block * sizeof(BndState<R>); }
+   // dynamic shared memory: a header and the boundary states of every lane of a block
+   static size_t smem(int slots, int block) { return kSmemHeader + (size_t)(slots > 0 ? slots : 1) * block * sizeof(BndState<R>); }
 
    // the guiding-centre family runs on static backgrounds only (no kernels for the moving shocks)
    template <int BG>

@@ -206,6 +206,8 @@ struct RunConfig {
    // 1 when a problem has a DistributionLossCone: the |B| extrema along each trajectory are tracked
    // (the reference's RECORD_BMAG_EXTREMA build, src/trajectory_base.cc:581-592)
    int track_bmag;
+   // the plain grid: lanes of a warp that hold trajectories, in teams of "team" lanes a trajectory (FP64)
+   int warp_lanes, team;
 };
 
 // Device-side counters of one run (scratch memory, zeroed before each launch).

@@ -21,6 +21,7 @@ constexpr uint32_t TRAJ_FINISH = 0x0010u, TRAJ_TIME_CROSSED = 0x0020u, TRAJ_SPAT
 constexpr uint32_t kMaxTrajSteps = 10000000u;  // src/trajectory_base.hh:38
 constexpr int kMaxBndTotal = 3 * kMaxBnd;
 
+constexpr size_t kSmemHeader = 16;  // dynamic shared memory: the team size, then the boundary states
 constexpr unsigned kErrAction = 1u;  // RunCounters::error: an action beyond the ActionTable
 
 // Lane state carried across steps.
@@ -53,6 +54,7 @@ struct Sinks {
    double* sums;
    unsigned long long* n_events;  // [problem * kMaxDistro + distro]
    RunCounters* ctr;
+   bool lead;  // the first lane of its team: events and counts are its own
 };
 
 template <class R, class A>
@@ -411,6 +413,7 @@ template <int TT, class R, class A>
 __device__ __forceinline__ void distro_events(const Lane<R, A>& L, const SD<R>& sp, const Start& s0,
                                               const ProblemDesc& Pd, int j, const Sinks& S)
 {
+   if (!S.lead) return;
    const BndParams& b = bnd_param(Pd, j);
    EventPoint e = event_point(L, sp);
    for (int di = 0; di < Pd.nd; di++) {
@@ -606,29 +609,35 @@ __device__ __forceinline__ bool prev_step_ok(Lane<R, A>& L, R dmax)
 }
 
 // ---- Parker (src/trajectory_parker.cc:83-306) ----------------------------------------------
-template <int BG, class R>
-__device__ __noinline__ bool parker_divk_fd(const ProblemDescT<R>& P, int deriv_mode, R t, V3<R> pos, R p, R vmag,
-                                            const SD<R>& sp, V3<R>& divK)
+template <int BG>
+__device__ __noinline__ bool parker_divk_fd(const ProblemDesc& P, int deriv_mode, double t, V3<double> pos, double p, double vmag,
+                                            const SD<double>& sp, V3<double>& divK)
 {
    // TRAJ_PARKER_DIVK_METHOD 0 (src/trajectory_parker.cc:87-119): central differences of the tensor
-   R delta = m_min(larmor(p, sp.Bmag), sp.dmax);
+   using R = double;
+   const R delta = m_min(larmor(p, sp.Bmag), sp.dmax);
+   const bool rigidity_b = P.df.kind == kDfRigidityB;
+   const R factor = rigidity_b ? kappa_rigidity_factor(P.df, p, vmag) : R(0);
+   R pts[6][3];
+   const bool ok = six_points<3>(pts, [&](int k, R (&v)[3]) {
+      const int j = k >> 1;
+      R x = pos[j] + delta;
+      if (k & 1) x -= R(2) * delta;
+      const V3<R> pt = mk(j == 0 ? x : pos.x, j == 1 ? x : pos.y, j == 2 ? x : pos.z);
+      SD<R> f;
+      if (!get_fields<BG>(P.bg, deriv_mode, t, pt, p, kU | kB, f)) return false;
+      const Kap<R> K = rigidity_b ? kappa_rigidity_b(P.df, factor, f.Bmag) : kappa_pp(P.df, pt, p, vmag, kap_in(f));
+      const R bj = f.bhat[j];
+#pragma unroll
+      for (int i = 0; i < 3; i++) v[i] = K.perp * (i == j ? R(1) : R(0)) + (K.para - K.perp) * bj * f.bhat[i];
+      return true;
+   });
+   if (!ok) return false;
+   const Divisor<R> over_delta(delta);
    R dk[3] = {R(0), R(0), R(0)};
-#pragma unroll 1
-   for (int j = 0; j < 3; j++) {
-      SD<R> sf, sb;
-      R pt[3] = {pos.x, pos.y, pos.z};
-      pt[j] = pt[j] + delta;
-      if (!get_fields<BG>(P.bg, deriv_mode, t, mk(pt[0], pt[1], pt[2]), p, kU | kB, sf)) return false;
-      Kap<R> kf = kappa_pp(P.df, mk(pt[0], pt[1], pt[2]), p, vmag, kap_in(sf));
-      pt[j] -= R(2) * delta;
-      if (!get_fields<BG>(P.bg, deriv_mode, t, mk(pt[0], pt[1], pt[2]), p, kU | kB, sb)) return false;
-      Kap<R> kb = kappa_pp(P.df, mk(pt[0], pt[1], pt[2]), p, vmag, kap_in(sb));
-      for (int i = 0; i < 3; i++) {
-         R f = kf.perp * (i == j ? R(1) : R(0)) + (kf.para - kf.perp) * sf.bhat[j] * sf.bhat[i];
-         R b = kb.perp * (i == j ? R(1) : R(0)) + (kb.para - kb.perp) * sb.bhat[j] * sb.bhat[i];
-         dk[i] += quot(R(0.5) * (f - b), delta);
-      }
-   }
+   for (int j = 0; j < 3; j++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) dk[i] += over_delta(R(0.5) * (pts[2 * j][i] - pts[2 * j + 1][i]));
    divK = mk(dk[0], dk[1], dk[2]);
    return true;
 }
@@ -644,10 +653,12 @@ __device__ __forceinline__ bool parker_slopes(const ProblemDescT<R>& P, int deri
    const R vmag = vel_of(p);
    K = kappa_pp(P.df, pos, p, vmag, kap_in(sp));
    V3<R> divK;
-   if (sizeof(R) == sizeof(double) && deriv_mode == 0) {
-      if (!parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) return false;
+   bool fd = false;
+   if constexpr (sizeof(R) == sizeof(double)) {
+      fd = deriv_mode == 0;
+      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) return false;
    }
-   else {
+   if (!fd) {
       V3<R> gpe, gpa;
       kappa_grad(P.df, pos, p, vmag, sp, K, gpe, gpa);
       V3<R> t1 = gpa - gpe;
@@ -678,6 +689,23 @@ __device__ __forceinline__ R parker_source(Lane<R, A>& L, const ProblemDescT<R>&
       L.src_del_old = del;
    }
    return sa;
+}
+
+// The normals of a Parker step: n[0] .. n[2]. A team's even lanes form the first Box-Muller pair, its odd
+// lanes the second.
+__device__ __forceinline__ void step_normals(uint4 b, float n[4]) { normals4<float>(b, n); }
+__device__ __forceinline__ void step_normals(uint4 b, double n[4])
+{
+   const Team tm = my_team();
+   if (tm.size == 1) { normals4<double>(b, n); return; }
+   const bool odd = tm.rank & 1;
+   const double r = m_sqrt(-2.0 * m_log(u01d(odd ? b.z : b.x)));
+   double s, c;
+   sincos_2pi(u01d(odd ? b.w : b.y), &s, &c);
+   const double v0 = r * c, v1 = r * s;
+   n[0] = tm.from(v0, 0);
+   n[1] = tm.from(v1, 0);
+   n[2] = tm.from(v0, 1);
 }
 
 // ---- Parker steps in a uniform field -----------------------------------------------------------
@@ -751,7 +779,7 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    const R sa = P.src.kind ? parker_source(L, P, (R)acc_val(L.mom.x), val3<R>(L.pos)) : R(0);
    L.dt = time_proximity(h.dtp, h.dmax, bv, n_time_bnd<BL>(P), fwd);
    R n[4];
-   normals4<R>(rng_block(P.seed, L.steps, L.traj_id, P.problem_id, kRngStep, L.attempt), n);
+   step_normals(rng_block(P.seed, L.steps, L.traj_id, P.problem_id, kRngStep, L.attempt), n);
    R sdt = m_sqrt(L.dt);
    R dWx = sdt * n[0], dWy = sdt * n[1], dWz = sdt * n[2];
    V3<R> dr = from_basis(mk(h.sperp * dWx, h.sperp * dWy, h.spara * dWz), h.fa);
@@ -814,10 +842,12 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    // DiffusionCoeff (src/trajectory_parker.cc:83-153)
    Kap<R> K = kappa_pp<R, DK>(P.df, pos, p, vmag, kap_in(sp));
    V3<R> divK;
-   if (kFP64 && deriv_mode == 0) {
-      if (!parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) { L.status |= TRAJ_DISCARD; return; }
+   bool fd = false;
+   if constexpr (kFP64) {
+      fd = deriv_mode == 0;
+      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) { L.status |= TRAJ_DISCARD; return; }
    }
-   else {
+   if (!fd) {
       // TRAJ_PARKER_DIVK_METHOD 1 (src/trajectory_parker.cc:120-140)
       V3<R> gpe, gpa;
       kappa_grad<R, false, DK>(P.df, pos, p, vmag, sp, K, gpe, gpa);
@@ -850,7 +880,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    L.dt = time_proximity(m_min(dtp, L.dt_adapt), sp.dmax, bv, n_time_bnd<BL>(P), fwd);
    // EulerDiffSlopes (src/trajectory_parker.cc:159-180)
    R n[4];
-   normals4<R>(rng_block(P.seed, L.steps, L.traj_id, P.problem_id, kRngStep, L.attempt), n);
+   step_normals(rng_block(P.seed, L.steps, L.traj_id, P.problem_id, kRngStep, L.attempt), n);
    R sdt = m_sqrt(L.dt);
    R sperp = m_sqrt(R(2) * K.perp), spara = m_sqrt(R(2) * K.para);
    // the reference's field-aligned basis (GetSecondUnitVec): n0, n1 across, n2 along the field
@@ -1653,9 +1683,14 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
 {
    using A = typename AccOf<R>::type;
    cfg.deriv_mode = DM;
-   extern __shared__ __align__(16) unsigned char spx_smem[];
-   const BndView<R> bv{reinterpret_cast<BndState<R>*>(spx_smem) + threadIdx.x, (int)blockDim.x};
-   Sinks S{counts, sums, n_events, ctr};
+   const BndView<R> bv{reinterpret_cast<BndState<R>*>(spx_smem + kSmemHeader) + threadIdx.x, (int)blockDim.x};
+   // a team of lanes shares a trajectory in the FP64 plain grid only
+   const int team = sizeof(R) == sizeof(double) && !queue ? cfg.team : 1;
+   if constexpr (sizeof(R) == sizeof(double)) {
+      if (threadIdx.x == 0) *reinterpret_cast<int*>(spx_smem) = team;
+      __syncthreads();
+   }
+   Sinks S{counts, sums, n_events, ctr, (threadIdx.x & (team - 1)) == 0};
    Lane<R, A> L;
    Start s0;
    [[maybe_unused]] UniformStep<R> held;
@@ -1666,10 +1701,13 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
    unsigned long long my_steps = 0;
    unsigned my_retries = 0, my_given_up = 0, my_done = 0;
    const int64_t total = cfg.total_traj;
-   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+   // the plain grid: a warp has cfg.warp_lanes lanes at work, in teams
+   const int lanes = queue ? 32 : cfg.warp_lanes, per_warp = lanes / team;
+   const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5) * per_warp;
    if (!queue) {
-      g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-      if (g < total) { active = true; fresh = true; }
+      const int lane = threadIdx.x & 31;
+      g = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane / team;
+      if (lane < lanes && g < total) { active = true; fresh = true; }
    }
    const int K = cfg.steps_per_sync > 0 ? cfg.steps_per_sync : 1;
    while (true) {
@@ -1701,11 +1739,11 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             // discarded attempt: redo the trajectory with a fresh random stream (src/simulation.cc:262-288)
             if (L.attempt + 1 >= (uint32_t)cfg.max_attempts) {
                L.status |= TRAJ_GAVE_UP;
-               my_given_up++;
+               if (S.lead) my_given_up++;
                done = true;
             }
             else {
-               my_retries++;
+               if (S.lead) my_retries++;
                attempt = L.attempt + 1;
                fresh = true;
                continue;
@@ -1728,7 +1766,7 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             done = (L.status & TRAJ_FINISH) && !(L.status & TRAJ_DISCARD);
             // timing samples of the autotuner stop every trajectory after a fixed number of steps
             if (cfg.step_cap && L.steps >= cfg.step_cap && !done) {
-               my_steps += L.steps;
+               if (S.lead) my_steps += L.steps;
                active = false;
                if (!queue) {
                   g += stride;
@@ -1738,9 +1776,11 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             }
          }
          if (done) {
-            my_steps += L.steps;
-            my_done++;
-            if (cfg.record_final) write_record(L, s0, rec, g);
+            if (S.lead) {
+               my_steps += L.steps;
+               my_done++;
+               if (cfg.record_final) write_record(L, s0, rec, g);
+            }
             active = false;
             if (!queue) {
                g += stride;

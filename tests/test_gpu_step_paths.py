@@ -2,6 +2,7 @@
 
 - Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
   1e140 takes the time-step bounds there (FP64 against the oracle).
+- Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
   and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
   kernels of one diffusion class against the kernel that dispatches at run time, whose steps are general."""
@@ -11,6 +12,7 @@ import pytest
 import oracle_tools as ot
 import test_oracle_plugins as cases
 from spectrum_gb300 import capi
+from spectrum_gb300 import workloads as W
 from spectrum_gb300.datacontainer import DataContainer as DC
 from spectrum_gb300.plugins import DiffusionRigidityMagneticFieldPowerLaw
 from spectrum_gb300.simulation import open_problems, run_problems
@@ -59,3 +61,24 @@ def test_quotients_outside_the_fast_range(built_lib):
     pb = cases._parker(n=40, bg=bg, t_end=0.1)
     res = run_problems(pb, precision=capi.SPX_FP64, record=True)
     ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
+
+
+@pytest.mark.parametrize("n", [1, 31, 700, 2433, 4865, 9729])
+@pytest.mark.parametrize("kind", ["modulation", "focused", "guiding"])
+def test_lane_teams_equal_single_lanes(built_lib, kind, n):
+    """Small FP64 launches give a trajectory several lanes (eight up to 2,432 trajectories, four, two, then one) and
+    spread over all schedulers; the launch shape given here has one lane each in full warps."""
+    if kind == "modulation":
+        pb = W.gcr_modulation(n_traj=n, energies_mev=[300.0], t_max_years=1.0e-4, pow_law_b=-1.0)[0]
+    elif kind == "focused":
+        pb = W.focused_transport(n_problems=1, n_traj=n, t_max_hours=0.002)[0]
+    else:
+        pb = W.guiding_dipole(n_traj=n, t_end_s=0.1)
+    a = run_problems(pb, precision=capi.SPX_FP64, record=True)
+    b = run_problems(pb, precision=capi.SPX_FP64, record=True, tuning=capi.Tuning(128, 0, 0, 0))
+    assert a.stats.trajectories == b.stats.trajectories == n and a.stats.steps == b.stats.steps > n
+    assert a.stats.events == b.stats.events
+    for f in ("attempts", "status", "steps", "t", "pos", "mom"):
+        assert np.array_equal(a.records[0][f], b.records[0][f]), f
+    for (ca, _, na), (cb, _, nb) in zip(a.distros[0], b.distros[0]):
+        assert na == nb and np.array_equal(ca, cb)
