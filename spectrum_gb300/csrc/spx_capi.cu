@@ -370,7 +370,7 @@ cudaError_t launch(spx_ctx* c, const spx::LaunchArgs& a)
    }
 }
 
-int occupancy(spx_ctx* c, int block, int slots)
+int occupancy(spx_ctx* c, int block, int slots, bool deep)
 {
    const bool f64 = c->precision == SPX_FP64, fd = f64 && c->deriv_mode == 0;
    const int bg = c->bg_kind;
@@ -378,43 +378,43 @@ int occupancy(spx_ctx* c, int block, int slots)
       switch (c->traj) {
       case SPX_TRAJ_PARKER:
       case SPX_TRAJ_PARKER_SOURCE:
-         return fd ? spx::occupancy_parker_f64fdrk(bg, block, slots) : spx::occupancy_parker_f64rk(bg, block, slots);
+         return fd ? spx::occupancy_parker_f64fdrk(bg, block, slots, deep) : spx::occupancy_parker_f64rk(bg, block, slots, deep);
       case SPX_TRAJ_LORENTZ:
-         return fd ? spx::occupancy_lorentz_f64fdrk(bg, block, slots) : spx::occupancy_lorentz_f64rk(bg, block, slots);
+         return fd ? spx::occupancy_lorentz_f64fdrk(bg, block, slots, deep) : spx::occupancy_lorentz_f64rk(bg, block, slots, deep);
       case SPX_TRAJ_FOCUSED:
-         return fd ? spx::occupancy_focused_f64fdrk(bg, block, slots) : spx::occupancy_focused_f64rk(bg, block, slots);
-      case SPX_TRAJ_FIELDLINE: return spx::occupancy_fieldline_f64rk(bg, block, slots);
+         return fd ? spx::occupancy_focused_f64fdrk(bg, block, slots, deep) : spx::occupancy_focused_f64rk(bg, block, slots, deep);
+      case SPX_TRAJ_FIELDLINE: return spx::occupancy_fieldline_f64rk(bg, block, slots, deep);
       default:
-         return fd ? spx::occupancy_guiding_f64fdrk(bg, block, slots) : spx::occupancy_guiding_f64rk(bg, block, slots);
+         return fd ? spx::occupancy_guiding_f64fdrk(bg, block, slots, deep) : spx::occupancy_guiding_f64rk(bg, block, slots, deep);
       }
    }
-   if (guiding_plain(c)) return spx::occupancy_guiding_f32p(bg, block, slots);
+   if (guiding_plain(c)) return spx::occupancy_guiding_f32p(bg, block, slots, deep);
    switch (parker_f32_special(c)) {
    case spx::kDfRigidityB:
-      return layout_spheres(c) ? spx::occupancy_parker_f32rbs(bg, block, slots) : spx::occupancy_parker_f32rb(bg, block, slots);
+      return layout_spheres(c) ? spx::occupancy_parker_f32rbs(bg, block, slots, deep) : spx::occupancy_parker_f32rb(bg, block, slots, deep);
    case spx::kDfFull:
-      return layout_spheres(c) ? spx::occupancy_parker_f32fcs(bg, block, slots) : spx::occupancy_parker_f32fc(bg, block, slots);
+      return layout_spheres(c) ? spx::occupancy_parker_f32fcs(bg, block, slots, deep) : spx::occupancy_parker_f32fc(bg, block, slots, deep);
    default: break;
    }
    switch (c->traj) {
    case SPX_TRAJ_PARKER:
    case SPX_TRAJ_PARKER_SOURCE:
-      return fd ? spx::occupancy_parker_f64fd(bg, block, slots)
-                : f64 ? spx::occupancy_parker_f64(bg, block, slots) : spx::occupancy_parker_f32(bg, block, slots);
+      return fd ? spx::occupancy_parker_f64fd(bg, block, slots, deep)
+                : f64 ? spx::occupancy_parker_f64(bg, block, slots, deep) : spx::occupancy_parker_f32(bg, block, slots, deep);
    case SPX_TRAJ_LORENTZ:
-      return fd ? spx::occupancy_lorentz_f64fd(bg, block, slots)
-                : f64 ? spx::occupancy_lorentz_f64(bg, block, slots) : spx::occupancy_lorentz_f32(bg, block, slots);
+      return fd ? spx::occupancy_lorentz_f64fd(bg, block, slots, deep)
+                : f64 ? spx::occupancy_lorentz_f64(bg, block, slots, deep) : spx::occupancy_lorentz_f32(bg, block, slots, deep);
    case SPX_TRAJ_FOCUSED:
-      return fd ? spx::occupancy_focused_f64fd(bg, block, slots)
-                : f64 ? spx::occupancy_focused_f64(bg, block, slots) : spx::occupancy_focused_f32(bg, block, slots);
+      return fd ? spx::occupancy_focused_f64fd(bg, block, slots, deep)
+                : f64 ? spx::occupancy_focused_f64(bg, block, slots, deep) : spx::occupancy_focused_f32(bg, block, slots, deep);
    case SPX_TRAJ_GUIDING:
    case SPX_TRAJ_GUIDING_SCATT:
    case SPX_TRAJ_GUIDING_DIFF:
    case SPX_TRAJ_GUIDING_DIFF_SCATT:
-      return fd ? spx::occupancy_guiding_f64fd(bg, block, slots)
-                : f64 ? spx::occupancy_guiding_f64(bg, block, slots) : spx::occupancy_guiding_f32(bg, block, slots);
+      return fd ? spx::occupancy_guiding_f64fd(bg, block, slots, deep)
+                : f64 ? spx::occupancy_guiding_f64(bg, block, slots, deep) : spx::occupancy_guiding_f32(bg, block, slots, deep);
    case SPX_TRAJ_FIELDLINE:
-      return f64 ? spx::occupancy_fieldline_f64(bg, block, slots) : spx::occupancy_fieldline_f32(bg, block, slots);
+      return f64 ? spx::occupancy_fieldline_f64(bg, block, slots, deep) : spx::occupancy_fieldline_f32(bg, block, slots, deep);
    default: return 0;
    }
 }
@@ -443,14 +443,27 @@ void set_rk(const spx_ctx* c, spx::RunConfig& cfg)
          if (p.pd.d[d].kind == spx::kDsLossCone) cfg.track_bmag = 1;
 }
 
+// Trajectories per lane of the deep build (58,368 lanes on a GB300) up to which an untuned FP32 run takes it.
+// Measured, wide against deep build: in a uniform field trajectories take the same steps and a launch has no
+// drain to speak of (3e4 trajectories 1.52 / 1.08 ms, 6e4 1.59 / 2.09, 1e6 15.3 / 18.2): one per lane. Lorentz
+// orbits in the dipole (2e5 42.3 / 39.8 ms, 4e5 60.3 / 63.2): five. Parker trajectories elsewhere differ in
+// length by a factor of ten and more, and the drain lasts as long as the longest (modulation, 1.9e5: 205 /
+// 143 ms, 1.28e6: 411 / 371; shock, 8e5: 151 / 148; grid, 6.4e5: 250 / 206): twenty.
+int64_t deep_lanes_limit(const spx_ctx* c)
+{
+   return c->traj == SPX_TRAJ_LORENTZ ? 5 : (c->bg_kind == spx::kBgUniform ? 1 : 20);
+}
+
 // The launch shape of a run: the caller's, else the one spx_autotune chose, else the defaults (the
 // FP64 drop-in keeps one thread per trajectory; the FP32 stepper takes the persistent queue in
-// blocks of 64 refilled every 8 steps, the shape that measured fastest on the modulation batch).
+// blocks of 64 refilled every 8 steps, the shape that measured fastest on the modulation batch, or up to
+// deep_lanes_limit the kernels' deep build in blocks of 128, whose warps it repacks).
 // Unset fields are completed and checked; blocks per SM is capped by the kernel's occupancy for
 // "slots" boundary states per lane. Shared by spx_run and spx_run_static.
-int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, spx_tuning& tu)
+int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t total, spx_tuning& tu, bool& deep)
 {
    tu = spx_tuning{};
+   deep = false;
    if (tuning) tu = *tuning;
    else if (c->has_tuned) tu = c->tuned;
    else {
@@ -458,13 +471,18 @@ int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, spx_tuning& 
       if (tu.schedule) {
          tu.block_size = 64;
          tu.steps_per_sync = 8;
+         const int occ = occupancy(c, 128, slots, true);
+         if (occ > 0 && total <= deep_lanes_limit(c) * c->sm_count * 128 * occ) {
+            deep = true;
+            tu.block_size = 128;
+         }
       }
    }
    if (tu.schedule != 0 && tu.schedule != 1) return SPX_ERR_INVALID_ARG;
    if (tu.block_size <= 0) tu.block_size = 128;
    if (tu.block_size % 32 || tu.block_size > 128) return SPX_ERR_INVALID_ARG;
    if (tu.steps_per_sync <= 0) tu.steps_per_sync = tu.schedule ? 16 : 1 << 30;
-   int occ = occupancy(c, tu.block_size, slots);
+   int occ = occupancy(c, tu.block_size, slots, deep);
    if (occ <= 0) occ = 1;
    if (tu.blocks_per_sm <= 0 || tu.blocks_per_sm > occ) tu.blocks_per_sm = occ;
    return SPX_OK;
@@ -503,7 +521,7 @@ PlainShape plain_shape(const spx_ctx* c, int64_t total, int block, bool chosen_h
 // index, and the device buffers. A different key means a new capture.
 struct GraphKey {
    unsigned grid, block, slots;
-   int queue;
+   int queue, deep;
    spx::RunConfig cfg;
    const void* ptr[7];
 };
@@ -517,6 +535,7 @@ void graph_key(const spx::LaunchArgs& a, unsigned char* out)
    k.block = a.block.x;
    k.slots = (unsigned)a.bnd_slots;
    k.queue = a.queue;
+   k.deep = a.deep;
    k.cfg = a.cfg;
    k.cfg.run_index = 0;
    const void* p[7] = {a.problems_r, a.problems_d, a.ctr, a.counts, a.sums, a.n_events, a.records};
@@ -955,9 +974,9 @@ int spx_run(spx_ctx_t c, const spx_tuning* tuning)
    }
    spx_tuning tu;
    const int slots = bnd_slots(c);
-   const int trc = resolve_tuning(c, tuning, slots, tu);
-   if (trc != SPX_OK) return trc;
    spx::LaunchArgs a;
+   const int trc = resolve_tuning(c, tuning, slots, c->total_traj, tu, a.deep);
+   if (trc != SPX_OK) return trc;
    const PlainShape ps = plain_shape(c, c->total_traj, tu.block_size, tuning == nullptr && !c->has_tuned);
    if (tu.schedule == 0) tu.block_size = ps.block;
    a.block = dim3(tu.block_size);
@@ -993,6 +1012,7 @@ int spx_run(spx_ctx_t c, const spx_tuning* tuning)
    a.records = c->d_rec;
    a.queue = tu.schedule;
    a.bnd_slots = slots;
+   a.cfg.bnd_slots = slots;
    if (c->record_final && c->d_rec == nullptr) return SPX_ERR_STATE;
    // trajectory ids of this run, run_index * n_traj ... (run_index + 1) * n_traj - 1, must fit 32 bits
    for (const auto& p : c->problems)
@@ -1078,12 +1098,13 @@ int spx_autotune(spx_ctx_t c, int64_t sample_traj, spx_tuning* best)
    double best_rate = -1.0;
    spx_tuning best_tu = cands[0];
    for (spx_tuning tu : cands) {
-      int occ = occupancy(c, tu.block_size, slots);
+      int occ = occupancy(c, tu.block_size, slots, false);
       if (occ <= 0) continue;
       tu.blocks_per_sm = occ;
       int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * occ : (first + tu.block_size - 1) / tu.block_size;
       spx::LaunchArgs a;
       a.block = dim3(tu.block_size);
+      a.deep = false;
       a.cfg.warp_lanes = 32;
       a.cfg.team = 1;
       a.grid = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff)));
@@ -1114,6 +1135,7 @@ int spx_autotune(spx_ctx_t c, int64_t sample_traj, spx_tuning* best)
       a.records = nullptr;
       a.queue = tu.schedule;
       a.bnd_slots = slots;
+      a.cfg.bnd_slots = slots;
       SPX_CUDA(cudaMemsetAsync(b_ctr.p, 0, sizeof(spx::RunCounters), c->stream));
       SPX_CUDA(cudaEventRecord(c->ev0, c->stream));
       SPX_CUDA(launch(c, a));
@@ -1612,7 +1634,8 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    // launch shape: chosen as spx_run chooses it (the caller's, the autotuned one, or the defaults)
    spx_tuning tu;
    const int slots = bnd_slots(c);
-   rc = resolve_tuning(c, tuning, slots, tu);
+   spx::LaunchArgs a;
+   rc = resolve_tuning(c, tuning, slots, total, tu, a.deep);
    if (rc != SPX_OK) return rc;
    const PlainShape ps = plain_shape(c, total, tu.block_size, tuning == nullptr && !c->has_tuned);
    if (tu.schedule == 0) tu.block_size = ps.block;
@@ -1632,7 +1655,6 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
       SPX_CUDA(cudaMemcpyAsync(scratch + off_pr, hf.data(), bytes_pr, cudaMemcpyHostToDevice, c->stream));
    }
 
-   spx::LaunchArgs a;
    a.block = dim3(tu.block_size);
    a.grid = dim3((unsigned)grid);
    a.cfg.warp_lanes = ps.warp_lanes;
@@ -1664,6 +1686,7 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    a.records = c->record_final ? reinterpret_cast<spx::TrajRecord*>(records) : nullptr;
    a.queue = tu.schedule;
    a.bnd_slots = slots;
+   a.cfg.bnd_slots = slots;
    SPX_CUDA(cudaEventRecord(c->ev0, c->stream));
    SPX_CUDA(launch(c, a));
    SPX_CUDA(cudaEventRecord(c->ev1, c->stream));

@@ -19,28 +19,44 @@ struct FamilyTU {
    template <int BG>
    static constexpr bool kBuilt = !(TT == kGuiding && (BG == kBgShock || BG == kBgSmoothShock));
 
-   template <int BG>
-   static cudaError_t go(const LaunchArgs& a)
+   // Parker and Lorentz in FP32 have the deep build too
+   static constexpr int kBlocks = sizeof(R) == 4 ? kWideBlocksF32 : kBlocksF64;
+   static constexpr bool kHasDeep = sizeof(R) == 4 && (TT == kParker || TT == kLorentz);
+
+   template <int BG, int MB>
+   static cudaError_t go_build(const LaunchArgs& a)
    {
-      if constexpr (kBuilt<BG>) {
-         const auto* P = static_cast<const ProblemDescT<R>*>(a.problems_r);
-         step_kernel<TT, BG, R, DM, GT, DK, BL><<<a.grid, a.block, smem(a.bnd_slots, a.block.x), a.stream>>>(
-             P, a.problems_d, a.cfg, a.ctr, a.counts, a.sums, a.n_events, a.records, a.queue);
-         return cudaGetLastError();
-      }
-      else return cudaErrorInvalidValue;
+      const auto* P = static_cast<const ProblemDescT<R>*>(a.problems_r);
+      step_kernel<TT, BG, R, DM, GT, DK, BL, MB><<<a.grid, a.block, smem(a.bnd_slots, a.block.x), a.stream>>>(
+          P, a.problems_d, a.cfg, a.ctr, a.counts, a.sums, a.n_events, a.records, a.queue);
+      return cudaGetLastError();
    }
 
    template <int BG>
-   static int occ(int block, int slots)
+   static cudaError_t go(const LaunchArgs& a)
+   {
+      if constexpr (!kBuilt<BG>) return cudaErrorInvalidValue;
+      else if constexpr (kHasDeep) return a.deep ? go_build<BG, kDeepBlocksF32>(a) : go_build<BG, kBlocks>(a);
+      else return go_build<BG, kBlocks>(a);
+   }
+
+   template <int BG, int MB>
+   static int occ_build(int block, int slots)
    {
       int n = 0;
-      if constexpr (kBuilt<BG>) {
-         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<TT, BG, R, DM, GT, DK, BL>, block, smem(slots, block)) !=
-             cudaSuccess)
-            n = 0;
-      }
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, step_kernel<TT, BG, R, DM, GT, DK, BL, MB>, block, smem(slots, block)) !=
+          cudaSuccess)
+         n = 0;
       return n;
+   }
+
+   // deep: the deep build's occupancy, 0 where there is none
+   template <int BG>
+   static int occ(int block, int slots, bool deep)
+   {
+      if constexpr (!kBuilt<BG>) return 0;
+      else if constexpr (kHasDeep) return deep ? occ_build<BG, kDeepBlocksF32>(block, slots) : occ_build<BG, kBlocks>(block, slots);
+      else return deep ? 0 : occ_build<BG, kBlocks>(block, slots);
    }
 
    static cudaError_t launch(int bg, const LaunchArgs& a)
@@ -56,15 +72,15 @@ struct FamilyTU {
       }
    }
 
-   static int occupancy(int bg, int block, int slots)
+   static int occupancy(int bg, int block, int slots, bool deep)
    {
       switch (bg) {
-      case kBgUniform: return occ<kBgUniform>(block, slots);
-      case kBgShock: return occ<kBgShock>(block, slots);
-      case kBgSmoothShock: return occ<kBgSmoothShock>(block, slots);
-      case kBgDipole: return occ<kBgDipole>(block, slots);
-      case kBgSolarWind: return occ<kBgSolarWind>(block, slots);
-      case kBgGrid: return occ<kBgGrid>(block, slots);
+      case kBgUniform: return occ<kBgUniform>(block, slots, deep);
+      case kBgShock: return occ<kBgShock>(block, slots, deep);
+      case kBgSmoothShock: return occ<kBgSmoothShock>(block, slots, deep);
+      case kBgDipole: return occ<kBgDipole>(block, slots, deep);
+      case kBgSolarWind: return occ<kBgSolarWind>(block, slots, deep);
+      case kBgGrid: return occ<kBgGrid>(block, slots, deep);
       default: return 0;
       }
    }
@@ -80,11 +96,11 @@ struct FamilyTU {
 #define SPX_FAMILY_TU_DK(fam, prec, TT, DK, BL)                                                                    \
    namespace spx {                                                                                                  \
    cudaError_t launch_##fam##_##prec(int bg, const LaunchArgs& a) { return FamilyTU<TT, float, 1, false, DK, BL>::launch(bg, a); } \
-   int occupancy_##fam##_##prec(int bg, int block, int slots) { return FamilyTU<TT, float, 1, false, DK, BL>::occupancy(bg, block, slots); } \
+   int occupancy_##fam##_##prec(int bg, int block, int slots, bool deep) { return FamilyTU<TT, float, 1, false, DK, BL>::occupancy(bg, block, slots, deep); } \
    }
 
 #define SPX_FAMILY_TU(fam, prec, TT, R, DM, GT)                                                                    \
    namespace spx {                                                                                                  \
    cudaError_t launch_##fam##_##prec(int bg, const LaunchArgs& a) { return FamilyTU<TT, R, DM, GT>::launch(bg, a); } \
-   int occupancy_##fam##_##prec(int bg, int block, int slots) { return FamilyTU<TT, R, DM, GT>::occupancy(bg, block, slots); } \
+   int occupancy_##fam##_##prec(int bg, int block, int slots, bool deep) { return FamilyTU<TT, R, DM, GT>::occupancy(bg, block, slots, deep); } \
    }

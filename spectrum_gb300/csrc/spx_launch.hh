@@ -22,6 +22,7 @@ struct LaunchArgs {
    TrajRecord* records;
    int queue;                       // 1: persistent work-queue schedule
    int bnd_slots;                   // boundary states per lane (the largest problem's count)
+   bool deep;                       // the FP32 kernels' deep build (three resident blocks per SM)
 };
 
 #define SPX_DECLARE_FAMILY(fam)                                        \
@@ -30,11 +31,11 @@ struct LaunchArgs {
    cudaError_t launch_##fam##_f32(int bg, const LaunchArgs& a);        \
    cudaError_t launch_##fam##_f64rk(int bg, const LaunchArgs& a);      \
    cudaError_t launch_##fam##_f64fdrk(int bg, const LaunchArgs& a);    \
-   int occupancy_##fam##_f64(int bg, int block, int slots);            \
-   int occupancy_##fam##_f64fd(int bg, int block, int slots);          \
-   int occupancy_##fam##_f32(int bg, int block, int slots);            \
-   int occupancy_##fam##_f64rk(int bg, int block, int slots);          \
-   int occupancy_##fam##_f64fdrk(int bg, int block, int slots);
+   int occupancy_##fam##_f64(int bg, int block, int slots, bool deep);            \
+   int occupancy_##fam##_f64fd(int bg, int block, int slots, bool deep);          \
+   int occupancy_##fam##_f32(int bg, int block, int slots, bool deep);            \
+   int occupancy_##fam##_f64rk(int bg, int block, int slots, bool deep);          \
+   int occupancy_##fam##_f64fdrk(int bg, int block, int slots, bool deep);
 SPX_DECLARE_FAMILY(parker)
 // the FP32 Parker kernels specialised for one diffusion class, and for it and the layout of one time
 // boundary and two spheres (kLayoutSpheres)
@@ -42,13 +43,13 @@ cudaError_t launch_parker_f32rb(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32fc(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32rbs(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32fcs(int bg, const LaunchArgs& a);
-int occupancy_parker_f32rb(int bg, int block, int slots);
-int occupancy_parker_f32fc(int bg, int block, int slots);
-int occupancy_parker_f32rbs(int bg, int block, int slots);
-int occupancy_parker_f32fcs(int bg, int block, int slots);
+int occupancy_parker_f32rb(int bg, int block, int slots, bool deep);
+int occupancy_parker_f32fc(int bg, int block, int slots, bool deep);
+int occupancy_parker_f32rbs(int bg, int block, int slots, bool deep);
+int occupancy_parker_f32fcs(int bg, int block, int slots, bool deep);
 // the FP32 guiding-centre kernels for TrajectoryGuiding proper (kDkNoDiffusion)
 cudaError_t launch_guiding_f32p(int bg, const LaunchArgs& a);
-int occupancy_guiding_f32p(int bg, int block, int slots);
+int occupancy_guiding_f32p(int bg, int block, int slots, bool deep);
 SPX_DECLARE_FAMILY(lorentz)
 SPX_DECLARE_FAMILY(focused)
 SPX_DECLARE_FAMILY(guiding)
@@ -57,8 +58,8 @@ SPX_DECLARE_FAMILY(guiding)
 cudaError_t launch_fieldline_f64(int bg, const LaunchArgs& a);
 cudaError_t launch_fieldline_f64rk(int bg, const LaunchArgs& a);
 cudaError_t launch_fieldline_f32(int bg, const LaunchArgs& a);
-int occupancy_fieldline_f64(int bg, int block, int slots);
-int occupancy_fieldline_f64rk(int bg, int block, int slots);
-int occupancy_fieldline_f32(int bg, int block, int slots);
+int occupancy_fieldline_f64(int bg, int block, int slots, bool deep);
+int occupancy_fieldline_f64rk(int bg, int block, int slots, bool deep);
+int occupancy_fieldline_f32(int bg, int block, int slots, bool deep);
 
 }  // namespace spx

@@ -208,6 +208,7 @@ struct RunConfig {
    int track_bmag;
    // the plain grid: lanes of a warp that hold trajectories, in teams of "team" lanes a trajectory (FP64)
    int warp_lanes, team;
+   int bnd_slots;             // boundary states per lane (the largest problem's count)
 };
 
 // Device-side counters of one run (scratch memory, zeroed before each launch).

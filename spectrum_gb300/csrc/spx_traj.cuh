@@ -874,7 +874,11 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
       L.src_del_old = del;
    }
    // PhysicalStep (src/trajectory_parker.cc:212-221)
-   R dtp = R(0.5) * sp.dmax / norm(slope);
+   R dtp;
+   // on a grid the wide and deep builds would fuse different products of the sum: it is fixed here
+   if constexpr (BG == kBgGrid && !kFP64)
+      dtp = R(0.5) * sp.dmax / m_sqrt(__fmaf_rn(slope.z, slope.z, __fmaf_rn(slope.y, slope.y, __fmul_rn(slope.x, slope.x))));
+   else dtp = R(0.5) * sp.dmax / norm(slope);
    dtp = m_min(dtp, R(0.5) * (sp.dmax * sp.dmax) / m_max(K.perp, K.para));
    dtp = m_min(dtp, R(0.5) * R(3) * R(0.01) / m_abs(divU));
    L.dt = time_proximity(m_min(dtp, L.dt_adapt), sp.dmax, bv, n_time_bnd<BL>(P), fwd);
@@ -1656,16 +1660,91 @@ __device__ __forceinline__ void start_lane(Lane<R, A>& L, BndView<R> bv, Start& 
    L.amp = n.amp; L.wgt = n.wgt; L.dt = n.dt; L.dt_adapt = n.dt_adapt; L.src_del_old = n.src_del_old;
 }
 
-// Resident blocks of 128 threads per SM the register allocation is sized for. For the FP32
-// kernels five blocks (20 warps, at most 102 registers) measured 2-5% faster than four blocks
-// without spills: the extra warps hide more dependent-instruction latency than the spilled
-// values cost.
-#ifndef SPX_MIN_BLOCKS_F32
-#define SPX_MIN_BLOCKS_F32 5
-#endif
-#ifndef SPX_MIN_BLOCKS_F64
-#define SPX_MIN_BLOCKS_F64 1
-#endif
+// ---- repacking the lanes of a block ----------------------------------------------------------
+// Once the queue is dry a block's trajectories only end, and the last of them sit in nearly every warp, a few
+// lanes each: as many warps issue as at the start, for a fraction of the steps. When the block's active lanes
+// fit in fewer warps, their states move to the first threads and the warps left empty wait at the block's
+// barrier, so the others have the schedulers (and in FP64 the pipe, which a warp occupies as long for one
+// lane as for 32). A block repacks at most blockDim / 32 - 1 times. Without it the deep build
+// took 499, 270 and 405 ms on the three runs given below, with it 453, 245 and 375.
+
+// Lane state as words, for the exchange below.
+struct LaneWords {
+   static constexpr int kMax = 48;
+   unsigned long long w[kMax];
+   int n;
+   template <class T> __device__ __forceinline__ void put(const T& v)
+   {
+      static_assert(sizeof(T) == 4 || sizeof(T) == 8, "lane state is made of 4- and 8-byte members");
+      unsigned long long u = 0;
+      memcpy(&u, &v, sizeof v);
+      w[n++] = u;
+   }
+   template <class T> __device__ __forceinline__ void get(T& v) { memcpy(&v, &w[n++], sizeof v); }
+};
+
+template <class R, class A, class F>
+__device__ __forceinline__ void each_member(Lane<R, A>& L, F f)
+{
+   f(L.prob); f(L.traj_id); f(L.attempt); f(L.steps); f(L.status); f(L.nrm); f(L.n_adapt);
+   f(L.t);
+   f(L.pos.x); f(L.pos.y); f(L.pos.z);
+   f(L.mom.x); f(L.mom.y); f(L.mom.z);
+   f(L.amp); f(L.wgt); f(L.dt); f(L.dt_adapt); f(L.src_del_old);
+}
+template <class R, class F>
+__device__ __forceinline__ void each_member(UniformStep<R>& h, F f)
+{
+   int valid = h.valid;
+   f(valid);
+   h.valid = valid != 0;
+   f(h.slope.x); f(h.slope.y); f(h.slope.z);
+   for (int k = 0; k < 3; k++) { f(h.fa[k].x); f(h.fa[k].y); f(h.fa[k].z); }
+   f(h.slope_p); f(h.sperp); f(h.spara); f(h.dtp); f(h.dmax); f(h.Bmag); f(h.divU);
+}
+
+// Moves the words and boundary states of the block's active lanes to its first threads, in order; every
+// thread of the block takes part. Returns whether this thread holds a trajectory afterwards.
+template <class R>
+__device__ __noinline__ bool repack_lanes(LaneWords& W, Start& s0, BndView<R> bv, int slots, bool active, unsigned long long* buf)
+{
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+   const unsigned mask = __ballot_sync(0xffffffffu, active);
+   if (lane == 0) buf[warp] = __popc(mask);
+   __syncthreads();
+   int rank = __popc(mask & ((1u << lane) - 1u)), total = 0;
+   for (int k = 0; k < (int)blockDim.x / 32; k++) {
+      const int c = (int)buf[k];
+      if (k < warp) rank += c;
+      total += c;
+   }
+   __syncthreads();
+   const bool mine = tid < total;
+   auto move = [&](unsigned long long& v) {
+      if (active) buf[rank] = v;
+      __syncthreads();
+      if (mine) v = buf[tid];
+      __syncthreads();
+   };
+   for (int k = 0; k < W.n; k++) move(W.w[k]);
+   static_assert(sizeof(Start) % 8 == 0, "Start is moved in 8-byte words");
+   for (int k = 0; k < (int)(sizeof(Start) / 8); k++) move(reinterpret_cast<unsigned long long*>(&s0)[k]);
+   for (int j = 0; j < slots; j++) {
+      const BndState<R> b = bv.ld(j);
+      __syncthreads();
+      if (active) (bv.p - tid)[j * bv.stride + rank] = b;
+   }
+   __syncthreads();
+   return mine;
+}
+
+// Resident blocks of 128 threads per SM the register allocation is sized for. The FP32 kernels come in two
+// builds. Wide, five blocks (20 warps, at most 102 registers), has the most steps per second with every lane
+// busy: the extra warps hide more dependent-instruction latency than the spilled values cost (four blocks ran
+// 2-5% slower). Deep, three blocks, spills nothing, so a warp's step is shorter: it is the faster one where a
+// launch is mostly its drain, the last trajectories alone on the SMs. One GB300, wide to deep with its repacking: shock acceleration of 4e4
+// trajectories 580 -> 453 ms, modulation of 1.9e5 325 -> 245 ms, on a 256^3 grid 530 -> 375 ms.
+constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
 
 // One lane per thread. Dynamic shared memory holds the lanes' boundary states
 // (boundaries per lane x blockDim.x x sizeof(BndState<R>)).
@@ -1676,8 +1755,13 @@ __device__ __forceinline__ void start_lane(Lane<R, A>& L, BndView<R> bv, Start& 
 // kDkNoDiffusion: the guiding-centre kernels for TrajectoryGuiding proper (no scattering, no perpendicular step).
 // BL: the boundary layout (BndLayout) the Parker step is compiled for; kLayoutAny reads it from the
 // descriptor.
-template <int TT, int BG, class R, int DM, bool GT, int DK, int BL>
-__global__ void __launch_bounds__(128, sizeof(R) == 4 ? SPX_MIN_BLOCKS_F32 : SPX_MIN_BLOCKS_F64)
+// MB: resident blocks of 128 per SM (above); the wide FP32 build does not repack its lanes.
+// Steps between two barriers of a draining block: few enough that a warp emptied early is soon given up,
+// enough that waiting for the slowest of the block's warps costs little.
+constexpr int kDrainSteps = 32;
+
+template <int TT, int BG, class R, int DM, bool GT, int DK, int BL, int MB>
+__global__ void __launch_bounds__(128, MB)
 step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict__ Pd, RunConfig cfg,
             RunCounters* ctr, int32_t* counts, double* sums, unsigned long long* n_events, TrajRecord* rec, int queue)
 {
@@ -1709,9 +1793,20 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
       g = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane / team;
       if (lane < lanes && g < total) { active = true; fresh = true; }
    }
-   const int K = cfg.steps_per_sync > 0 ? cfg.steps_per_sync : 1;
+   // The plain grid drains from the start. The queue's lanes refill until a warp of the block finds it dry;
+   // then the block's warps go on together: K steps, a barrier, and a repacking where it empties a warp.
+   constexpr bool kRepack = MB != kWideBlocksF32;
+   __shared__ unsigned long long s_buf[kRepack ? 128 : 1];
+   __shared__ volatile int s_dry;
+   if constexpr (kRepack) {
+      if (threadIdx.x == 0) s_dry = !queue;
+      __syncthreads();
+   }
+   [[maybe_unused]] bool drain = false;
+   [[maybe_unused]] int live = blockDim.x >> 5;  // warps that may hold trajectories
+   int K = cfg.steps_per_sync > 0 ? cfg.steps_per_sync : 1;
    while (true) {
-      if (queue) {
+      if (queue && !drain) {
          // refill idle lanes from the work queue: one atomic per warp
          unsigned idle = __ballot_sync(0xffffffffu, !active);
          if (idle) {
@@ -1723,8 +1818,39 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             if (!active) {
                int64_t mine = (int64_t)base + __popc(idle & ((1u << lane) - 1u));
                if (mine < total) { g = mine; active = true; fresh = true; attempt = 0; }
+               else if constexpr (kRepack) s_dry = 1;
             }
          }
+      }
+      if constexpr (kRepack) {
+         if (!drain && __any_sync(0xffffffffu, s_dry != 0)) {
+            drain = true;
+            K = kDrainSteps;
+         }
+         if (drain) {
+            const int n = __syncthreads_count(active);
+            if (n == 0) break;
+            const int need = (n + 31) >> 5;
+            if (need < live) {
+               live = need;
+               LaneWords W;
+               W.n = 0;
+               auto put = [&](auto& v) { W.put(v); };
+               each_member(L, put);
+               if constexpr (TT == kParker && holds_uniform_step<BG, DK, R>()) each_member(held, put);
+               int flag = fresh;
+               put(g); put(attempt); put(flag);
+               active = repack_lanes(W, s0, bv, cfg.bnd_slots, active, s_buf);
+               W.n = 0;
+               auto get = [&](auto& v) { W.get(v); };
+               each_member(L, get);
+               if constexpr (TT == kParker && holds_uniform_step<BG, DK, R>()) each_member(held, get);
+               get(g); get(attempt); get(flag);
+               fresh = flag != 0;
+            }
+         }
+      }
+      else if (queue) {
          if (!__any_sync(0xffffffffu, active)) break;
       }
       else if (!active) break;

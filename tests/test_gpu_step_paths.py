@@ -2,6 +2,7 @@
 
 - Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
   1e140 takes the time-step bounds there (FP64 against the oracle).
+- The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
   and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
@@ -11,7 +12,7 @@ import pytest
 
 import oracle_tools as ot
 import test_oracle_plugins as cases
-from spectrum_gb300 import capi
+from spectrum_gb300 import capi, units
 from spectrum_gb300 import workloads as W
 from spectrum_gb300.datacontainer import DataContainer as DC
 from spectrum_gb300.plugins import DiffusionRigidityMagneticFieldPowerLaw
@@ -82,3 +83,29 @@ def test_lane_teams_equal_single_lanes(built_lib, kind, n):
         assert np.array_equal(a.records[0][f], b.records[0][f]), f
     for (ca, _, na), (cb, _, nb) in zip(a.distros[0], b.distros[0]):
         assert na == nb and np.array_equal(ca, cb)
+
+
+@pytest.mark.parametrize("n", [1, 33, 129, 4097, 60_001])
+@pytest.mark.parametrize("kind", ["uniform", "spiral", "shock", "grid", "dipole"])
+def test_deep_build_equals_the_wide_one(built_lib, kind, n):
+    """Untuned FP32 runs of few trajectories a lane take the kernels' deep build, whose blocks repack their lanes as
+    trajectories end; a given launch shape takes the wide build. The same trajectories, bit for bit."""
+    if kind == "uniform":
+        pbs = [W.diffusion_uniform(n_traj=min(n, 50_000), t_end=0.02)]
+    elif kind == "spiral":  # two problems of different length, retries and both exits
+        pbs = W.gcr_modulation(n_traj=(n + 1) // 2, energies_mev=[30.0, 1000.0], t_max_years=0.005, pow_law_b=-1.0)
+    elif kind == "shock":
+        pbs = [W.shock_acceleration(n_traj=n, width_frac=0.2, x_escape=-0.3, x_downstream=0.3, p_max=2.0)]
+    elif kind == "grid":
+        pbs = W.gcr_modulation_grid(n_traj=n, n_nodes=32, energies_mev=[300.0], t_max_years=0.005)
+    else:
+        pbs = [W.dipole_orbits(n_traj=n, t_end=0.05 / units.unit_time)]
+    a = run_problems(pbs, precision=capi.SPX_MIXED, record=True)
+    b = run_problems(pbs, precision=capi.SPX_MIXED, record=True, tuning=capi.Tuning(64, 0, 8, 1))
+    assert a.stats.tuning.block_size == 128 and a.stats.steps == b.stats.steps and a.stats.retries == b.stats.retries
+    for ra, rb in zip(a.records, b.records):
+        for f in ("attempts", "status", "steps", "t", "pos", "mom", "pos0", "mom0"):
+            assert np.array_equal(ra[f], rb[f]), f
+    for da, db in zip(a.distros, b.distros):
+        for (ca, _, na), (cb, _, nb) in zip(da, db):
+            assert na == nb and np.array_equal(ca, cb)
