@@ -45,6 +45,7 @@ struct SD {
    M3<R> gradU, gradB;
    R Bmag, dmax, divU, divbhat;
    R dr[3];
+   V3<R> fa0, fa1;  // across the field, from numerical_derivs (the basis is fa0, fa1, bhat)
 };
 
 template <class R> __device__ __forceinline__ R sd_divU(const SD<R>& s) { return s.divU; }
@@ -531,7 +532,7 @@ __device__ __forceinline__ bool grid_fields(const BgParamsT<R>& g, V3<R> pos, un
 // with the same numbers. They share out the points of finite differences and the halves of a Box-Muller
 // block: the FP64 pipe takes as long for one lane as for 32, so a launch too small to fill the lanes has
 // them for nothing. One GB300: 1,200 modulation trajectories with numerical
-// derivatives 855 -> 307 ms in teams of eight.
+// derivatives 855 -> 307 ms in teams of eight, 254 ms with the rows of the gradients shared out as well.
 extern __shared__ __align__(16) unsigned char spx_smem[];
 struct Team {
    int size, rank;
@@ -544,27 +545,27 @@ __device__ __forceinline__ Team my_team()
    return {size, lane & (size - 1), ((size < 32 ? (1u << size) : 0u) - 1u) << (lane & ~(size - 1))};
 }
 
-// Central differences evaluate six points, forward and backward along three axes. point(k, v) evaluates
-// point k (axis k / 2, backward if odd) into v[0 .. N) and returns whether it could; the team's lanes take
-// a point each, and every lane gets all of them in out. Returns false if a point failed, on all lanes alike.
-template <int N, class F>
-__device__ __forceinline__ bool six_points(double (&out)[6][N], F point)
+// M pieces of work of N results each, shared out over the team: piece(k, v) puts piece k into v[0 .. N) and returns
+// whether it could; a lane takes pieces rank, rank + size, ... and every lane gets them all in out. Returns
+// false if a piece failed, on all lanes alike.
+template <int M, int N, class F>
+__device__ __forceinline__ bool team_share(double (&out)[M][N], F piece)
 {
    const Team tm = my_team();
    bool ok = true;
 #pragma unroll 1
-   for (int k0 = 0; k0 < 6; k0 += tm.size) {
+   for (int k0 = 0; k0 < M; k0 += tm.size) {
       double v[N];
       const int k = k0 + tm.rank;
 #pragma unroll
       for (int i = 0; i < N; i++) v[i] = 0.0;
-      if (k < 6) ok = point(k, v) && ok;
+      if (k < M) ok = piece(k, v) && ok;
       if (tm.size == 1) {
 #pragma unroll
          for (int i = 0; i < N; i++) out[k][i] = v[i];
       }
       else {
-         for (int r = 0; r < tm.size && k0 + r < 6; r++)
+         for (int r = 0; r < tm.size && k0 + r < M; r++)
 #pragma unroll
             for (int i = 0; i < N; i++) out[k0 + r][i] = tm.from(v[i], r);
       }
@@ -581,19 +582,16 @@ __device__ __noinline__ void numerical_derivs(const BgParamsT<double>& g, double
    using R = double;
    unsigned m1 = mask >> 4, m2 = m1 >> 4;
    if (m1 & kAll) {
-      R r_g = m_min(larmor(p, s.Bmag), s.dmax);
-      V3<R> fa[3];
-      fa[2] = s.bhat;
-      fa[0] = second_unit(s.bhat);
-      fa[1] = cross(fa[2], fa[0]);
-      M3<R> gu, gbv;
-      R gbm[3];
+      const R r_g = m_min(larmor(p, s.Bmag), s.dmax);
+      s.fa0 = second_unit(s.bhat);
+      s.fa1 = cross(s.bhat, s.fa0);
+      // the six points, forward and backward along the axes of the field-aligned basis
       R pts[6][7];
       const R dr = r_g * R(2);
-      six_points<7>(pts, [&](int k, R (&v)[7]) {
+      team_share(pts, [&](int k, R (&v)[7]) {
          SD<R> f;
          R ds = R(0);
-         const V3<R> ax = k < 2 ? fa[0] : (k < 4 ? fa[1] : fa[2]);
+         const V3<R> ax = k < 2 ? s.fa0 : (k < 4 ? s.fa1 : s.bhat);
          V3<R> pt = pos + r_g * ax;
          if (k & 1) pt = pt - dr * ax;
          eval_bg<BG>(g, t, pt, m1, f, ds);
@@ -601,31 +599,30 @@ __device__ __noinline__ void numerical_derivs(const BgParamsT<double>& g, double
          if (m1 & kB) { v[3] = f.B.x; v[4] = f.B.y; v[5] = f.B.z; v[6] = norm(f.B); }
          return true;
       });
-      const Divisor<R> over_dr(dr);
+      // differences along each axis (U, B, |B|), then the rows of the gradients in the global frame
+      R q[3][7], rows[3][7];
+      team_share(q, [&](int k, R (&v)[7]) {
+         const Divisor<R> over_dr(dr);
 #pragma unroll
-      for (int xyz = 0; xyz < 3; xyz++) {
-         const R* f = pts[2 * xyz];
-         const R* b = pts[2 * xyz + 1];
-         if (m1 & kU)
-            for (int j = 0; j < 3; j++) gu.m[xyz][j] = over_dr(f[j] - b[j]);
-         if (m1 & kB) {
-            for (int j = 0; j < 3; j++) gbv.m[xyz][j] = over_dr(f[3 + j] - b[3 + j]);
-            gbm[xyz] = over_dr(f[6] - b[6]);
-         }
-         s.dr[xyz] = dr;
-      }
+         for (int j = 0; j < 7; j++) v[j] = over_dr(pts[2 * k][j] - pts[2 * k + 1][j]);
+         return true;
+      });
+      team_share(rows, [&](int i, R (&v)[7]) {
+         const R f0 = s.fa0[i], f1 = s.fa1[i], f2 = s.bhat[i];
 #pragma unroll
-      for (int i = 0; i < 3; i++)
+         for (int j = 0; j < 7; j++) v[j] = f0 * q[0][j] + f1 * q[1][j] + f2 * q[2][j];
+         return true;
+      });
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+         s.dr[i] = dr;
 #pragma unroll
          for (int j = 0; j < 3; j++) {
-            if (m1 & kU) s.gradU.m[i][j] = fa[0][i] * gu.m[0][j] + fa[1][i] * gu.m[1][j] + fa[2][i] * gu.m[2][j];
-            if (m1 & kB) s.gradB.m[i][j] = fa[0][i] * gbv.m[0][j] + fa[1][i] * gbv.m[1][j] + fa[2][i] * gbv.m[2][j];
+            if (m1 & kU) s.gradU.m[i][j] = rows[i][j];
+            if (m1 & kB) s.gradB.m[i][j] = rows[i][3 + j];
          }
-      if (m1 & kB) {
-         s.gradBmag = mk(fa[0].x * gbm[0] + fa[1].x * gbm[1] + fa[2].x * gbm[2],
-                         fa[0].y * gbm[0] + fa[1].y * gbm[1] + fa[2].y * gbm[2],
-                         fa[0].z * gbm[0] + fa[1].z * gbm[1] + fa[2].z * gbm[2]);
       }
+      if (m1 & kB) s.gradBmag = mk(rows[0][6], rows[1][6], rows[2][6]);
    }
    if (m2 & kAll) {
       R v = vel_of(p);
@@ -867,6 +864,13 @@ __device__ __forceinline__ R kappa_mumu_dmu(const DiffParamsT<R>& d, V3<R> pos, 
    if (d.kind != kDfQLT && d.kind != kDfWNLT && d.kind != kDfWNLTRamp) return R(0);
    R dmu = Lim<R>::small * (mu + Lim<R>::small < R(1) ? R(1) : R(-1));
    return (kappa_mumu(d, pos, vmag, Omega, mu + dmu) - dmumu) / dmu;
+}
+
+// Whether kappa_pp of the class reads the flow velocity.
+template <class R>
+__device__ __forceinline__ bool kappa_reads_flow(const DiffParamsT<R>& d)
+{
+   return d.kind == kDfFlowMomentum || d.kind == kDfKinEnergyRadial;
 }
 
 // Models whose gradient needs no field-gradient matrix (only grad|B| or grad U . U).

@@ -609,23 +609,35 @@ __device__ __forceinline__ bool prev_step_ok(Lane<R, A>& L, R dmax)
 }
 
 // ---- Parker (src/trajectory_parker.cc:83-306) ----------------------------------------------
+// kappa_pp at the step's point, with the momentum's factor kept for the difference points.
+__device__ __forceinline__ Kap<double> kappa_with_factor(const DiffParams& d, V3<double> pos, double p, double vmag,
+                                                         const SD<double>& sp, double& factor)
+{
+   factor = 0.0;
+   if (d.kind != kDfRigidityB) return kappa_pp(d, pos, p, vmag, kap_in(sp));
+   factor = kappa_rigidity_factor(d, p, vmag);
+   return kappa_rigidity_b(d, factor, sp.Bmag);
+}
+
+// "factor": kappa_rigidity_factor at this momentum, for that class.
 template <int BG>
 __device__ __noinline__ bool parker_divk_fd(const ProblemDesc& P, int deriv_mode, double t, V3<double> pos, double p, double vmag,
-                                            const SD<double>& sp, V3<double>& divK)
+                                            const SD<double>& sp, double factor, V3<double>& divK)
 {
    // TRAJ_PARKER_DIVK_METHOD 0 (src/trajectory_parker.cc:87-119): central differences of the tensor
    using R = double;
    const R delta = m_min(larmor(p, sp.Bmag), sp.dmax);
    const bool rigidity_b = P.df.kind == kDfRigidityB;
-   const R factor = rigidity_b ? kappa_rigidity_factor(P.df, p, vmag) : R(0);
+   const unsigned mask = kB | (kappa_reads_flow(P.df) ? kU : 0u);
    R pts[6][3];
-   const bool ok = six_points<3>(pts, [&](int k, R (&v)[3]) {
+   const bool ok = team_share(pts, [&](int k, R (&v)[3]) {
       const int j = k >> 1;
       R x = pos[j] + delta;
       if (k & 1) x -= R(2) * delta;
       const V3<R> pt = mk(j == 0 ? x : pos.x, j == 1 ? x : pos.y, j == 2 ? x : pos.z);
       SD<R> f;
-      if (!get_fields<BG>(P.bg, deriv_mode, t, pt, p, kU | kB, f)) return false;
+      f.U = mk(R(0), R(0), R(0));
+      if (!get_fields<BG>(P.bg, deriv_mode, t, pt, p, mask, f)) return false;
       const Kap<R> K = rigidity_b ? kappa_rigidity_b(P.df, factor, f.Bmag) : kappa_pp(P.df, pt, p, vmag, kap_in(f));
       const R bj = f.bhat[j];
 #pragma unroll
@@ -633,12 +645,15 @@ __device__ __noinline__ bool parker_divk_fd(const ProblemDesc& P, int deriv_mode
       return true;
    });
    if (!ok) return false;
-   const Divisor<R> over_delta(delta);
-   R dk[3] = {R(0), R(0), R(0)};
-   for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) dk[i] += over_delta(R(0.5) * (pts[2 * j][i] - pts[2 * j + 1][i]));
-   divK = mk(dk[0], dk[1], dk[2]);
+   R dk[3][1];
+   team_share(dk, [&](int i, R (&v)[1]) {
+      const Divisor<R> over_delta(delta);
+      R sum = R(0);
+      for (int j = 0; j < 3; j++) sum += over_delta(R(0.5) * (pts[2 * j][i] - pts[2 * j + 1][i]));
+      v[0] = sum;
+      return true;
+   });
+   divK = mk(dk[0][0], dk[1][0], dk[2][0]);
    return true;
 }
 
@@ -651,13 +666,15 @@ __device__ __forceinline__ bool parker_slopes(const ProblemDescT<R>& P, int deri
                                               const SD<R>& sp, bool fwd, Kap<R>& K, V3<R>& slope, R& slope_p)
 {
    const R vmag = vel_of(p);
-   K = kappa_pp(P.df, pos, p, vmag, kap_in(sp));
    V3<R> divK;
    bool fd = false;
    if constexpr (sizeof(R) == sizeof(double)) {
+      R factor;
+      K = kappa_with_factor(P.df, pos, p, vmag, sp, factor);
       fd = deriv_mode == 0;
-      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) return false;
+      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, factor, divK)) return false;
    }
+   else K = kappa_pp(P.df, pos, p, vmag, kap_in(sp));
    if (!fd) {
       V3<R> gpe, gpa;
       kappa_grad(P.df, pos, p, vmag, sp, K, gpe, gpa);
@@ -840,13 +857,16 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    track_bmag(s0, cfg, sp);
    R vmag = vel_of(p);
    // DiffusionCoeff (src/trajectory_parker.cc:83-153)
-   Kap<R> K = kappa_pp<R, DK>(P.df, pos, p, vmag, kap_in(sp));
+   Kap<R> K;
    V3<R> divK;
    bool fd = false;
    if constexpr (kFP64) {
+      R factor;
+      K = kappa_with_factor(P.df, pos, p, vmag, sp, factor);
       fd = deriv_mode == 0;
-      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, divK)) { L.status |= TRAJ_DISCARD; return; }
+      if (fd && !parker_divk_fd<BG>(P, deriv_mode, t, pos, p, vmag, sp, factor, divK)) { L.status |= TRAJ_DISCARD; return; }
    }
+   else K = kappa_pp<R, DK>(P.df, pos, p, vmag, kap_in(sp));
    if (!fd) {
       // TRAJ_PARKER_DIVK_METHOD 1 (src/trajectory_parker.cc:120-140)
       V3<R> gpe, gpa;
@@ -890,8 +910,14 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    // the reference's field-aligned basis (GetSecondUnitVec): n0, n1 across, n2 along the field
    V3<R> fa[3];
    fa[2] = sp.bhat;
-   fa[0] = second_unit(sp.bhat);
-   fa[1] = cross(fa[2], fa[0]);
+   if (kFP64 && BG == kBgSolarWind && fd) {  // numerical_derivs has formed them
+      fa[0] = sp.fa0;
+      fa[1] = sp.fa1;
+   }
+   else {
+      fa[0] = second_unit(sp.bhat);
+      fa[1] = cross(fa[2], fa[0]);
+   }
    R dWx = sdt * n[0], dWy = sdt * n[1], dWz = sdt * n[2];
    V3<R> dr = from_basis(mk(sperp * dWx, sperp * dWy, spara * dWz), fa);
    // RKStep with the Euler table, then the stochastic displacement
