@@ -239,14 +239,26 @@ static __device__ __noinline__ V3<double> sample_mom(InitRng& rng, const Problem
 // ---- distribution events (DistributionBase::ProcessTrajectory, src/distribution_base.cc:174-194;
 // DistributionTemplated::AddEvent, src/distribution_templated.cc:145-181), in FP64 ----------
 // The event's "second point" is the current state; its spatial data are the fields of the
-// step's start point, as in the reference (HandleBoundaries runs before CommonFields).
+// step's start point, as in the reference (HandleBoundaries runs before CommonFields). It is kept as the
+// kernel has it and turned into doubles where an event reads it: in the FP32 kernels every conversion
+// holds the FP64 pipe, and a guiding-centre orbit bins a mirror point every hundred steps (1e5 orbits of ten
+// seconds: 38.4 -> 36.5 ms; an event with no weight also leaves out the exponential).
+template <class R, class A>
 struct EventPoint {
-   double t;
-   V3<double> pos, mom, bhat;
-   double divU, amp, wgt, bmag;
+   A t_;
+   AV3<A> pos_, mom_;
+   V3<R> bhat_;
+   R divU_, amp_, wgt_, bmag_;
+   __device__ __forceinline__ double t() const { return acc_dbl(t_); }
+   __device__ __forceinline__ V3<double> pos() const { return mk(acc_dbl(pos_.x), acc_dbl(pos_.y), acc_dbl(pos_.z)); }
+   __device__ __forceinline__ V3<double> mom() const { return mk(acc_dbl(mom_.x), acc_dbl(mom_.y), acc_dbl(mom_.z)); }
+   __device__ __forceinline__ V3<double> bhat() const { return mk((double)bhat_.x, (double)bhat_.y, (double)bhat_.z); }
+   __device__ __forceinline__ double divU() const { return (double)divU_; }
+   __device__ __forceinline__ double bmag() const { return (double)bmag_; }
 };
 
-static __device__ __noinline__ void process_event(int traj, const EventPoint& e, const Start& s0, const ProblemDesc& P,
+template <class R, class A>
+__device__ __noinline__ void process_event(int traj, const EventPoint<R, A>& e, const Start& s0, const ProblemDesc& P,
                                            int prob, int di, int action, const Sinks& S)
 {
    const DistParams& d = P.d[di];
@@ -257,9 +269,9 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
    V3<double> value = mk(0.0, 0.0, 0.0);
    double w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
    switch (d.kind) {
-   case kDsTimeUniform: value.x = d.val_time == 0 ? s0.t0 : e.t; break;
+   case kDsTimeUniform: value.x = d.val_time == 0 ? s0.t0 : e.t(); break;
    case kDsPositionUniform: case kDsLossCone:
-      value = d.val_time == 0 ? s0.pos0 : e.pos;
+      value = d.val_time == 0 ? s0.pos0 : e.pos();
       if (d.val_coord == 1) {  // Metric<SphericalRTP>::PosToCurv, common/coordinates.hh:124-135
          double r = norm(value), phi = atan2(value.y, value.x);
          if (phi < 0.0) phi += 6.283185307179586476925286766559;
@@ -267,8 +279,8 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
       }
       break;
    case kDsMomentumUniform: {
-      V3<double> m = d.val_time == 0 ? s0.mom0 : e.mom;
-      V3<double> bh = d.val_time == 0 ? s0.bhat0 : e.bhat;
+      V3<double> m = d.val_time == 0 ? s0.mom0 : e.mom();
+      V3<double> bh = d.val_time == 0 ? s0.bhat0 : e.bhat();
       if (d.val_coord == 0 || (traj != kLorentz && traj != kGuiding && traj != kFieldline)) value = m;
       else if (traj == kFieldline) value = mk(m.z, 0.0, 0.0);  // src/distribution_other.cc:276-279
       else if (traj == kLorentz) { double mm = norm(m); value = mk(mm, dot(m, bh) / mm, 0.0); }
@@ -276,7 +288,7 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
       break;
    }
    case kDsPositionMomentumUniform: {
-      V3<double> p = d.val_time == 0 ? s0.pos0 : e.pos, m = d.val_time == 0 ? s0.mom0 : e.mom;
+      V3<double> p = d.val_time == 0 ? s0.pos0 : e.pos(), m = d.val_time == 0 ? s0.mom0 : e.mom();
       value.x = d.pos_idx == 3 ? norm(p) : p[d.pos_idx];
       value.y = m[d.mom_idx];
       break;
@@ -286,11 +298,11 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
       value.x = enr_kin<double>((traj == kLorentz || traj == kGuiding) ? norm(s0.mom0)
                                 : (traj == kFieldline ? s0.mom0.z : s0.mom0.x));
       break;
-   case kDsCumulative1: case kDsCumulative2: value.x = e.t; break;
+   case kDsCumulative1: case kDsCumulative2: value.x = e.t(); break;
    case kDsDivergenceFlow: value = s0.mom0; break;
    case kDsTimeMu:
-      value.x = e.t;
-      value.y = traj == kLorentz ? dot(e.mom, e.bhat) / norm(e.mom) : traj == kGuiding ? e.mom.z / norm(e.mom) : e.mom.y;
+      value.x = e.t();
+      value.y = traj == kLorentz ? dot(e.mom(), e.bhat()) / norm(e.mom()) : traj == kGuiding ? e.mom().z / norm(e.mom()) : e.mom().y;
       break;
    case kDsAnisotropyLISM: {  // EvaluateValue, src/distribution_other.cc:416-426
       // the first point's momentum in the binning frame, as (theta, phi) of its direction; the
@@ -312,32 +324,32 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
       break;
    case kDsSpectrumPowerLaw: case kDsSpectrumBentPowerLaw:
       if (action == 0) {  // DISTRO_KINETIC_ENERGY_POWER_LAW_TYPE 0, src/distribution_other.cc:567-591
-         double m2 = (traj == kLorentz || traj == kGuiding) ? norm(e.mom) : (traj == kFieldline ? e.mom.z : e.mom.x);
+         double m2 = (traj == kLorentz || traj == kGuiding) ? norm(e.mom()) : (traj == kFieldline ? e.mom().z : e.mom().x);
          double ke = enr_kin<double>(m2), v = vel_of<double>(m2);
          w[0] = d.J0 * v * pow(ke / d.T0, d.pow_law) / (m2 * m2);
          if (d.kind == kDsSpectrumBentPowerLaw) w[0] /= pow(1.0 + pow(ke / d.T_b, d.pow_law_comb), d.bend);
       }
       else w[0] = d.val_cold;
       break;
-   case kDsCumulative1: { V3<double> dp = e.pos - s0.pos0; w[0] = dp.x; w[1] = dp.y; w[2] = dp.z; break; }
+   case kDsCumulative1: { V3<double> dp = e.pos() - s0.pos0; w[0] = dp.x; w[1] = dp.y; w[2] = dp.z; break; }
    case kDsCumulative2: {
-      V3<double> dp = e.pos - s0.pos0;
+      V3<double> dp = e.pos() - s0.pos0;
       for (int i = 0; i < 3; i++)
          for (int j = 0; j < 3; j++) w[3 * i + j] = dp[i] * dp[j];
       break;
    }
-   case kDsDivergenceFlow: w[0] = action == 0 ? d.A0 * pow(fabs(e.divU), d.pow_law) : d.val_cold; break;
+   case kDsDivergenceFlow: w[0] = action == 0 ? d.A0 * pow(fabs(e.divU()), d.pow_law) : d.val_cold; break;
    case kDsLossCone:  // DistributionLossCone::RecordLossCone, src/distribution_other.cc:858-862
       w[0] = s0.bmag_min;
       w[1] = s0.bmag_max;
-      w[2] = asin(sqrt((d.val_time == 0 ? s0.bmag0 : e.bmag) / s0.bmag_max));
+      w[2] = asin(sqrt((d.val_time == 0 ? s0.bmag0 : e.bmag()) / s0.bmag_max));
       break;
    case kDsAnisotropyLISM: {  // the five anisotropy weights, src/distribution_other.cc:433-483
       const V3<double> ul = mk(d.u_lism[0], d.u_lism[1], d.u_lism[2]);
-      const double m1 = norm(s0.mom0), m2 = norm(e.mom);
+      const double m1 = norm(s0.mom0), m2 = norm(e.mom());
       // the second point's momentum in the LISM frame: p - gamma m U (RelFactor1, common/physics.hh:260-263)
       const double rf = sqrt(1.0 + (m2 / 1.0 / c_code<double>()) * (m2 / 1.0 / c_code<double>()));
-      const V3<double> rel = e.mom - (rf * 1.0) * ul;
+      const V3<double> rel = e.mom() - (rf * 1.0) * ul;
       const double rn = norm(rel);
       const V3<double> ru = mk(rel.x / rn, rel.y / rn, rel.z / rn);
       if (action == 0) {  // Compton-Getting factor
@@ -345,12 +357,12 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
          w[0] = 1.0 - dot(d.pow_law * ul, mh) / vel_of<double>(m1);
       }
       else if (action == 1) w[0] = pow(rn / m1, d.pow_law);
-      else if (action == 2) w[0] = dot(ru, e.bhat);
-      else if (action == 3) { const double c = dot(ru, e.bhat); w[0] = 0.5 * (3.0 * (c * c) - 1.0); }
+      else if (action == 2) w[0] = dot(ru, e.bhat());
+      else if (action == 3) { const double c = dot(ru, e.bhat()); w[0] = 0.5 * (3.0 * (c * c) - 1.0); }
       else {  // b x gradient: the guiding centre dotted with the density gradient
          const V3<double> gp = mk(d.grad_perp[0], d.grad_perp[1], d.grad_perp[2]);
-         const double rl = rn * c_code<double>() / (fabs(1.0) * e.bmag);
-         w[0] = dot(gp, e.pos + rl * cross(ru, e.bhat));
+         const double rl = rn * c_code<double>() / (fabs(1.0) * e.bmag());
+         w[0] = dot(gp, e.pos() + rl * cross(ru, e.bhat()));
       }
       break;
    }
@@ -380,25 +392,30 @@ static __device__ __noinline__ void process_event(int traj, const EventPoint& e,
       bin[k] = q <= -1.0 ? 0 : (int)q;
    }
    int64_t lin = (int64_t)d.n_bins[2] * ((int64_t)d.n_bins[1] * bin[0] + bin[1]) + bin[2];
-   double ew = exp(e.wgt);
-   for (int k = 0; k < d.width; k++) atomicAdd(&S.sums[d.offset_sums + lin * d.width + k], w[k] * ew + e.amp);
+   if (e.wgt_ == R(0) && e.amp_ == R(0)) {
+      for (int k = 0; k < d.width; k++) atomicAdd(&S.sums[d.offset_sums + lin * d.width + k], w[k]);
+   }
+   else {
+      const double ew = exp((double)e.wgt_), amp = (double)e.amp_;
+      for (int k = 0; k < d.width; k++) atomicAdd(&S.sums[d.offset_sums + lin * d.width + k], w[k] * ew + amp);
+   }
    atomicAdd(&S.counts[d.offset_counts + lin], 1);
    atomicAdd(&S.n_events[(int64_t)prob * kMaxDistro + di], 1ull);
    atomicAdd(&S.ctr->events, 1ull);  // the run's total, for spx_stats
 }
 
 template <class R, class A>
-__device__ __forceinline__ EventPoint event_point(const Lane<R, A>& L, const SD<R>& sp)
+__device__ __forceinline__ EventPoint<R, A> event_point(const Lane<R, A>& L, const SD<R>& sp)
 {
-   EventPoint e;
-   e.t = acc_dbl(L.t);
-   e.pos = mk(acc_dbl(L.pos.x), acc_dbl(L.pos.y), acc_dbl(L.pos.z));
-   e.mom = mk(acc_dbl(L.mom.x), acc_dbl(L.mom.y), acc_dbl(L.mom.z));
-   e.bhat = mk((double)sp.bhat.x, (double)sp.bhat.y, (double)sp.bhat.z);
-   e.divU = (double)sd_divU(sp);
-   e.bmag = (double)sp.Bmag;
-   e.amp = (double)L.amp;
-   e.wgt = (double)L.wgt;
+   EventPoint<R, A> e;
+   e.t_ = L.t;
+   e.pos_ = L.pos;
+   e.mom_ = L.mom;
+   e.bhat_ = sp.bhat;
+   e.divU_ = sd_divU(sp);
+   e.amp_ = L.amp;
+   e.wgt_ = L.wgt;
+   e.bmag_ = sp.Bmag;
    return e;
 }
 
@@ -415,7 +432,7 @@ __device__ __forceinline__ void distro_events(const Lane<R, A>& L, const SD<R>& 
 {
    if (!S.lead) return;
    const BndParams& b = bnd_param(Pd, j);
-   EventPoint e = event_point(L, sp);
+   EventPoint<R, A> e = event_point(L, sp);
    for (int di = 0; di < Pd.nd; di++) {
       int action = di < b.n_actions ? b.actions[di] : -1;
       if (action >= 0) process_event(TT, e, s0, Pd, L.prob, di, action, S);
