@@ -315,21 +315,33 @@ bool guiding_plain(const spx_ctx* c)
           !c->pa_scattering;
 }
 
-// Whether every problem has the boundary layout spx::kLayoutSpheres: one expiry or pass time boundary,
-// two spheres, no momentum boundary.
-bool layout_spheres(const spx_ctx* c)
+// The boundary layout (spx::BndLayout) of a problem, or kLayoutAny: one expiry or pass time boundary, and two
+// spheres, two planes with an injection or pass momentum boundary, or nothing else.
+int problem_layout(const spx::ProblemDesc& d)
 {
-   if (c->specialize != 1 || c->problems.empty()) return false;
-   for (const auto& p : c->problems) {
-      const spx::ProblemDesc& d = p.pd;
-      if (d.nbt != 1 || d.nbs != 2 || d.nbm != 0) return false;
-      if ((d.bt[0].kind != spx::kBtTimeExpire && d.bt[0].kind != spx::kBtTimePass) || d.bt[0].recurrent) return false;
-      for (int i = 0; i < 2; i++) {
-         const int k = d.bs[i].kind;
-         if (k != spx::kBtSphereAbsorb && k != spx::kBtSphereReflect && k != spx::kBtSpherePass) return false;
-      }
+   if (d.nbt != 1 || (d.bt[0].kind != spx::kBtTimeExpire && d.bt[0].kind != spx::kBtTimePass) || d.bt[0].recurrent) return spx::kLayoutAny;
+   if (d.nbs == 0 && d.nbm == 0) return spx::kLayoutTime;
+   if (d.nbs != 2) return spx::kLayoutAny;
+   int spheres = 0, planes = 0;
+   for (int i = 0; i < 2; i++) {
+      const int k = d.bs[i].kind;
+      spheres += k == spx::kBtSphereAbsorb || k == spx::kBtSphereReflect || k == spx::kBtSpherePass;
+      planes += k == spx::kBtPlaneAbsorb || k == spx::kBtPlaneReflect || k == spx::kBtPlanePass;
    }
-   return true;
+   if (spheres == 2 && d.nbm == 0) return spx::kLayoutSpheres;
+   if (planes == 2 && d.nbm == 1 && (d.bm[0].kind == spx::kBtMomentumInject || d.bm[0].kind == spx::kBtMomentumPass))
+      return spx::kLayoutPlanes;
+   return spx::kLayoutAny;
+}
+
+// The layout that every problem of the context has.
+int layout(const spx_ctx* c)
+{
+   if (c->specialize != 1 || c->problems.empty()) return spx::kLayoutAny;
+   const int first = problem_layout(c->problems[0].pd);
+   for (const auto& p : c->problems)
+      if (problem_layout(p.pd) != first) return spx::kLayoutAny;
+   return first;
 }
 
 cudaError_t launch(spx_ctx* c, const spx::LaunchArgs& a)
@@ -348,8 +360,14 @@ cudaError_t launch(spx_ctx* c, const spx::LaunchArgs& a)
    }
    if (guiding_plain(c)) return spx::launch_guiding_f32p(bg, a);
    switch (parker_f32_special(c)) {
-   case spx::kDfRigidityB: return layout_spheres(c) ? spx::launch_parker_f32rbs(bg, a) : spx::launch_parker_f32rb(bg, a);
-   case spx::kDfFull: return layout_spheres(c) ? spx::launch_parker_f32fcs(bg, a) : spx::launch_parker_f32fc(bg, a);
+   case spx::kDfRigidityB: return layout(c) == spx::kLayoutSpheres ? spx::launch_parker_f32rbs(bg, a) : spx::launch_parker_f32rb(bg, a);
+   case spx::kDfFull:
+      switch (layout(c)) {
+      case spx::kLayoutSpheres: return spx::launch_parker_f32fcs(bg, a);
+      case spx::kLayoutPlanes: return spx::launch_parker_f32fcp(bg, a);
+      case spx::kLayoutTime: return spx::launch_parker_f32fct(bg, a);
+      default: return spx::launch_parker_f32fc(bg, a);
+      }
    default: break;
    }
    switch (c->traj) {
@@ -391,9 +409,15 @@ int occupancy(spx_ctx* c, int block, int slots, bool deep)
    if (guiding_plain(c)) return spx::occupancy_guiding_f32p(bg, block, slots, deep);
    switch (parker_f32_special(c)) {
    case spx::kDfRigidityB:
-      return layout_spheres(c) ? spx::occupancy_parker_f32rbs(bg, block, slots, deep) : spx::occupancy_parker_f32rb(bg, block, slots, deep);
+      return layout(c) == spx::kLayoutSpheres ? spx::occupancy_parker_f32rbs(bg, block, slots, deep)
+                                              : spx::occupancy_parker_f32rb(bg, block, slots, deep);
    case spx::kDfFull:
-      return layout_spheres(c) ? spx::occupancy_parker_f32fcs(bg, block, slots, deep) : spx::occupancy_parker_f32fc(bg, block, slots, deep);
+      switch (layout(c)) {
+      case spx::kLayoutSpheres: return spx::occupancy_parker_f32fcs(bg, block, slots, deep);
+      case spx::kLayoutPlanes: return spx::occupancy_parker_f32fcp(bg, block, slots, deep);
+      case spx::kLayoutTime: return spx::occupancy_parker_f32fct(bg, block, slots, deep);
+      default: return spx::occupancy_parker_f32fc(bg, block, slots, deep);
+      }
    default: break;
    }
    switch (c->traj) {

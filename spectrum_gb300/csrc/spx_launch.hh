@@ -37,16 +37,20 @@ struct LaunchArgs {
    int occupancy_##fam##_f64rk(int bg, int block, int slots, bool deep);          \
    int occupancy_##fam##_f64fdrk(int bg, int block, int slots, bool deep);
 SPX_DECLARE_FAMILY(parker)
-// the FP32 Parker kernels specialised for one diffusion class, and for it and the layout of one time
-// boundary and two spheres (kLayoutSpheres)
+// the FP32 Parker kernels specialised for one diffusion class, and for it and a boundary layout
+// (kLayoutSpheres; for the constant class kLayoutPlanes and kLayoutTime too)
 cudaError_t launch_parker_f32rb(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32fc(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32rbs(int bg, const LaunchArgs& a);
 cudaError_t launch_parker_f32fcs(int bg, const LaunchArgs& a);
+cudaError_t launch_parker_f32fcp(int bg, const LaunchArgs& a);
+cudaError_t launch_parker_f32fct(int bg, const LaunchArgs& a);
 int occupancy_parker_f32rb(int bg, int block, int slots, bool deep);
 int occupancy_parker_f32fc(int bg, int block, int slots, bool deep);
 int occupancy_parker_f32rbs(int bg, int block, int slots, bool deep);
 int occupancy_parker_f32fcs(int bg, int block, int slots, bool deep);
+int occupancy_parker_f32fcp(int bg, int block, int slots, bool deep);
+int occupancy_parker_f32fct(int bg, int block, int slots, bool deep);
 // the FP32 guiding-centre kernels for TrajectoryGuiding proper (kDkNoDiffusion)
 cudaError_t launch_guiding_f32p(int bg, const LaunchArgs& a);
 int occupancy_guiding_f32p(int bg, int block, int slots, bool deep);

@@ -1015,12 +1015,11 @@ __device__ V3<R> bnd_normal(const BndParamsT<R>& b, V3<R> pos)
 // EvaluateBoundary (src/boundary_time.cc, src/boundary_space.cc, src/boundary_momentum.cc), one
 // evaluator per boundary class so that a loop over the boundaries of one class dispatches over that
 // class's kinds only. For time boundaries the delta is formed from the accumulated time.
-// BL 1: the boundary layout fixed at compile time (one expiry or pass time boundary and spheres, see
-// BndLayout); its evaluators skip the other kinds.
+// BL: the boundary layout fixed at compile time (BndLayout); its evaluators skip the other kinds.
 template <int BL, class R, class A>
 __device__ __forceinline__ void eval_time_bnd(const BndParamsT<R>& b, BndState<R>& st, const A& t)
 {
-   if (BL != 1 && b.kind == kBtTimeRecurrent) {
+   if (BL == kLayoutAny && b.kind == kBtTimeRecurrent) {
       R k = (R)((b.max_crossings - st.crossings_left) + 1);
       st.delta = (R)acc_diff(t, k * b.timemark, k * b.timemark_lo);
    }
@@ -1030,15 +1029,17 @@ __device__ __forceinline__ void eval_time_bnd(const BndParamsT<R>& b, BndState<R
 template <int BL, class R>
 __device__ __forceinline__ void eval_space_bnd(const BndParamsT<R>& b, BndState<R>& st, V3<R> pos, V3<R> region)
 {
-   // spheres first: the usual inner and outer boundaries of the heliospheric set-ups
-   if (BL == 1 || b.kind == kBtSphereAbsorb || b.kind == kBtSphereReflect || b.kind == kBtSpherePass) {
+   // spheres and planes first, one bit test each: the usual boundaries of the heliospheric and shock set-ups
+   const unsigned kind = BL == kLayoutSpheres || BL == kLayoutPlanes ? 0u : 1u << b.kind;
+   if (BL == kLayoutSpheres || (kind & (1u << kBtSphereAbsorb | 1u << kBtSphereReflect | 1u << kBtSpherePass))) {
       st.delta = norm(pos - ld3(b.origin)) - b.radius;
       return;
    }
-   switch (b.kind) {
-   case kBtPlaneAbsorb: case kBtPlaneReflect: case kBtPlanePass:
+   if (BL == kLayoutPlanes || (kind & (1u << kBtPlaneAbsorb | 1u << kBtPlaneReflect | 1u << kBtPlanePass))) {
       st.delta = dot(pos - ld3(b.origin), ld3(b.norm));
-      break;
+      return;
+   }
+   switch (b.kind) {
    case kBtBoxReflect: {
       st.delta = -Lim<R>::large;
 #pragma unroll
@@ -1067,10 +1068,14 @@ __device__ __forceinline__ void eval_space_bnd(const BndParamsT<R>& b, BndState<
    }
 }
 
-template <class R>
+template <int BL, class R>
 __device__ __forceinline__ void eval_mom_bnd(const BndParamsT<R>& b, BndState<R>& st, V3<R> pos, V3<R> mom,
                                              V3<R> bhat, int traj)
 {
+   if constexpr (BL == kLayoutPlanes) {  // Parker: an injection or pass boundary
+      st.delta = mom.x - b.momentum;
+      return;
+   }
    // BoundaryMirror::EvaluateBoundary (src/boundary_momentum.cc:329-339): the parallel momentum, which is
    // p mu for Focused, the native third component for the guiding-centre types and p . bhat for Lorentz
    if (b.kind == kBtMirror) {
@@ -1095,7 +1100,7 @@ __device__ __forceinline__ void eval_bnd(const BndParamsT<R>& b, BndState<R>& st
    const int cls = CLS >= 0 ? CLS : b.cls;
    if (cls == 0) eval_time_bnd<BL>(b, st, t);
    else if (cls == 1) eval_space_bnd<BL>(b, st, pos, region);
-   else eval_mom_bnd(b, st, pos, mom, bhat, traj);
+   else eval_mom_bnd<BL>(b, st, pos, mom, bhat, traj);
 }
 
 // BoundaryBase::ResetBoundary (src/boundary_base.cc:138-162)

@@ -519,9 +519,14 @@ __device__ __forceinline__ void handle_crossings(Lane<R, A>& L, BndView<R> bv, c
 // (RecordBoundary only copies delta to delta_old for it); crossed ones after their events.
 // Boundary counts per class: from the descriptor, or constants of the layout the kernel is compiled for
 // (the loops below then unroll).
-template <int BL, class R> __device__ __forceinline__ int n_time_bnd(const ProblemDescT<R>& P) { return BL == kLayoutSpheres ? 1 : P.nbt; }
-template <int BL, class R> __device__ __forceinline__ int n_space_bnd(const ProblemDescT<R>& P) { return BL == kLayoutSpheres ? 2 : P.nbs; }
-template <int BL, class R> __device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL == kLayoutSpheres ? 0 : P.nbm; }
+template <int BL, class R> __device__ __forceinline__ int n_time_bnd(const ProblemDescT<R>& P) { return BL == kLayoutAny ? P.nbt : 1; }
+template <int BL, class R>
+__device__ __forceinline__ int n_space_bnd(const ProblemDescT<R>& P)
+{
+   return BL == kLayoutAny ? P.nbs : (BL == kLayoutTime ? 0 : 2);
+}
+template <int BL, class R>
+__device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL == kLayoutAny ? P.nbm : (BL == kLayoutPlanes ? 1 : 0); }
 
 template <int TT, int BL, class R, class A>
 __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, const SD<R>& sp, const Start& s0,
@@ -569,7 +574,7 @@ __device__ __forceinline__ bool space_terminate(Lane<R, A>& L, BndView<R> bv, co
       const int j = P.nbt + i;
       BndState<R> b = bv.ld(j);
       compute_bnd<1>(P.bs[i], b, L.t, pos, mom, sp.bhat, sp.region, TT);
-      bv.st(j, b);
+      // (the state stays as it was: the step's end evaluates it again before anything reads it)
       if (b.crossed && b.crossings_left == 1) {
          L.status |= TRAJ_SPATIAL_CROSSED | TRAJ_FINISH;
          distro_events<TT>(L, sp, s0, Pd, j, S);

@@ -2,6 +2,7 @@
 
 - Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
   1e140 takes the time-step bounds there (FP64 against the oracle).
+- The FP32 kernels compiled for a boundary layout against the one that reads it from the descriptor.
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
@@ -109,3 +110,31 @@ def test_deep_build_equals_the_wide_one(built_lib, kind, n):
     for da, db in zip(a.distros, b.distros):
         for (ca, _, na), (cb, _, nb) in zip(da, db):
             assert na == nb and np.array_equal(ca, cb)
+
+
+@pytest.mark.parametrize("n", [1, 1000])
+@pytest.mark.parametrize("kind", ["absorbing_planes", "reflecting_planes_momentum_pass", "time_only"])
+def test_boundary_layout_kernels_equal_the_generic_one(built_lib, kind, n):
+    """The FP32 Parker kernels compiled for two planes with a momentum boundary, and for a time boundary alone,
+    against the kernel that reads kinds and counts from the descriptor: crossings of every boundary among them."""
+    c = cases
+    if kind == "absorbing_planes":
+        pb = W.shock_acceleration(n_traj=n, width_frac=0.1, x_escape=-0.3, x_downstream=0.3, p_max=1.2)
+    elif kind == "reflecting_planes_momentum_pass":
+        pb = c._parker(n=n, bg=c._shock(), t_end=0.3,
+                       bnds=[(c.BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((0.2, 0, 0)).vec((1.0, 0, 0))),
+                             (c.BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((-0.2, 0, 0)).vec((-1.0, 0, 0))),
+                             (c.BoundaryMomentumPass(), c.B(DC(), -1, [0]).double(1.01))])
+    else:
+        pb = W.diffusion_uniform(n_traj=n, t_end=0.1)
+    out = []
+    for special in (0, 1):
+        sim = open_problems(pb, precision=capi.SPX_MIXED, record=True)
+        sim.ctx.set_option(capi.SPX_OPT_SPECIALIZE, float(special))
+        st = sim.MainLoop()
+        out.append((st.events, sim.ctx.records(0, n), sim.ctx.distribution(0, 0)))
+        sim.close()
+    assert out[0][0] == out[1][0] and out[0][2][2] == out[1][2][2]
+    for f in ("status", "steps", "t", "pos", "mom"):
+        assert np.array_equal(out[0][1][f], out[1][1][f]), f
+    assert np.array_equal(out[0][2][0], out[1][2][0])
