@@ -41,6 +41,9 @@ __device__ __forceinline__ float m_max(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ void m_sincospi(double x, double* s, double* c) { sincospi(x, s, c); }
 __device__ __forceinline__ void m_sincospi(float x, float* s, float* c) { sincospif(x, s, c); }
 
+__device__ __forceinline__ double sub_down(double a, double b) { return __dsub_rd(a, b); }
+__device__ __forceinline__ float sub_down(float a, float b) { return __fsub_rd(a, b); }
+
 template <class R> struct Lim;
 template <> struct Lim<double> {
    static constexpr double large = 1.0E+20;
@@ -111,6 +114,7 @@ template <class R> __device__ __forceinline__ V3<R> operator/(V3<R> a, R s) { co
 template <class R> __device__ __forceinline__ R dot(V3<R> a, V3<R> b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 template <class R> __device__ __forceinline__ R norm2(V3<R> a) { return a.x * a.x + a.y * a.y + a.z * a.z; }
 template <class R> __device__ __forceinline__ R norm(V3<R> a) { return m_sqrt(norm2(a)); }
+template <class R> __device__ __forceinline__ R norm1(V3<R> a) { return m_abs(a.x) + m_abs(a.y) + m_abs(a.z); }
 template <class R> __device__ __forceinline__ V3<R> cross(V3<R> a, V3<R> b)
 {
    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};

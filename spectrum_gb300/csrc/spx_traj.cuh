@@ -36,6 +36,7 @@ struct Lane {
    AV3<A> pos, mom;  // mom: Parker (p,-,-), Focused (p, mu, -), Lorentz (px, py, pz), Guiding (p_perp, -, p_para),
                      // Fieldline (-, -, p_para)
    R amp, wgt, dt, dt_adapt, src_del_old;
+   R clear;  // within this distance of the point no spatial boundary is crossed (0: not known)
 };
 
 // Initial point of the trajectory (needed only by events and records).
@@ -528,9 +529,13 @@ __device__ __forceinline__ int n_space_bnd(const ProblemDescT<R>& P)
 template <int BL, class R>
 __device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL == kLayoutAny ? P.nbm : (BL == kLayoutPlanes ? 1 : 0); }
 
-template <int TT, int BL, class R, class A>
+// moved() is no less than the distance moved since the last call: while the clearance lasts no spatial
+// boundary can have been crossed, and none is evaluated (a state's delta_old is then an older one of the same sign;
+// of an absorbing or passing boundary only the sign is read). One GB300: focused transport 326 -> 286 ms, shock
+// acceleration 286 -> 268 ms, modulation 245 -> 238 ms.
+template <int TT, int BL, class R, class A, class F>
 __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, const SD<R>& sp, const Start& s0,
-                                                  const ProblemDescT<R>& P, const ProblemDesc& Pd, const Sinks& S)
+                                                  const ProblemDescT<R>& P, const ProblemDesc& Pd, const Sinks& S, F moved)
 {
    V3<R> pos = val3<R>(L.pos), mom = lane_mom(L);
    unsigned crossed = 0;
@@ -543,14 +548,28 @@ __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, 
       else b.delta_old = b.delta;
       bv.st(j, b);
    }
-   for (int i = 0; i < nbs; i++) {
-      const int j = nbt + i;
-      BndState<R> b = bv.ld(j);
-      compute_bnd<1, BL>(P.bs[i], b, L.t, pos, mom, sp.bhat, sp.region, TT);
-      if (b.crossed) crossed |= 1u << j;
-      else b.delta_old = b.delta;
-      bv.st(j, b);
+   if (nbs > 0) {
+      L.clear = sub_down(L.clear, moved() * R(1.0001));
+      if (!(L.clear > Lim<R>::tiny)) {
+         R clear = Lim<R>::large;
+         bool reflect = false;
+         const R reach = norm1(pos);
+         for (int i = 0; i < nbs; i++) {
+            const int j = nbt + i;
+            BndState<R> b = bv.ld(j);
+            compute_bnd<1, BL>(P.bs[i], b, L.t, pos, mom, sp.bhat, sp.region, TT);
+            if (b.crossed) crossed |= 1u << j;
+            else b.delta_old = b.delta;
+            bv.st(j, b);
+            clear = m_min(clear, bnd_clearance<BL>(P.bs[i], b.delta, reach));
+            reflect = reflect || P.bs[i].reflect;
+         }
+         // a reflection reads the last delta: its boundary is evaluated at every step's end (a negative clearance
+         // holds for the stage points only)
+         L.clear = crossed ? R(0) : (reflect ? -clear : clear);
+      }
    }
+   else L.clear = Lim<R>::large;
    for (int i = 0; i < nbm; i++) {
       const int j = nbt + nbs + i;
       BndState<R> b = bv.ld(j);
@@ -824,13 +843,16 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    V3<R> dr = from_basis(mk(h.sperp * dWx, h.sperp * dWy, h.spara * dWz), h.fa);
    R dts = L.dt * R(1);
    acc_add(L.t, fwd ? L.dt : -L.dt);
+   V3<R> d;
    if constexpr (kFP64) {
-      const R sgn = fwd ? dts : -dts;
-      acc_add(L.pos.x, sgn * h.slope.x); acc_add(L.pos.y, sgn * h.slope.y); acc_add(L.pos.z, sgn * h.slope.z);
-      acc_add(L.pos.x, dr.x); acc_add(L.pos.y, dr.y); acc_add(L.pos.z, dr.z);
+      d = (fwd ? dts : -dts) * h.slope;
+      add3(L.pos, d);
+      add3(L.pos, dr);
    }
-   else if (fwd) add3(L.pos, dts * h.slope + dr);
-   else add3(L.pos, dr - dts * h.slope);
+   else {
+      d = fwd ? dts * h.slope + dr : dr - dts * h.slope;
+      add3(L.pos, d);
+   }
    // -p div U / 3 is a zero, unless the momentum is not finite
    if (h.slope_p != R(0)) acc_add(L.mom.x, fwd ? dts * h.slope_p : -(dts * h.slope_p));
    if (sa != R(0)) L.amp += dts * sa * m_exp(L.wgt);
@@ -839,7 +861,7 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    sp.region = mk(R(1), R(1), R(1));
    sp.Bmag = h.Bmag;
    sp.divU = h.divU;
-   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S);
+   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
    L.steps++;
 }
 
@@ -944,32 +966,37 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    V3<R> dr = from_basis(mk(sperp * dWx, sperp * dWy, spara * dWz), fa);
    // RKStep with the Euler table, then the stochastic displacement
    R dts = L.dt * R(1);
+   V3<R> d;
    if (fwd) {
       acc_add(L.t, L.dt);
       if constexpr (kFP64) {
-         acc_add(L.pos.x, dts * slope.x); acc_add(L.pos.y, dts * slope.y); acc_add(L.pos.z, dts * slope.z);
+         d = dts * slope;
+         add3(L.pos, d);
          acc_add(L.mom.x, dts * slope_p);
-         acc_add(L.pos.x, dr.x); acc_add(L.pos.y, dr.y); acc_add(L.pos.z, dr.z);
+         add3(L.pos, dr);
       }
       else {
-         add3(L.pos, dts * slope + dr);
+         d = dts * slope + dr;
+         add3(L.pos, d);
          acc_add(L.mom.x, dts * slope_p);
       }
    }
    else {
       acc_add(L.t, -L.dt);
       if constexpr (kFP64) {
-         acc_add(L.pos.x, -(dts * slope.x)); acc_add(L.pos.y, -(dts * slope.y)); acc_add(L.pos.z, -(dts * slope.z));
+         d = (-dts) * slope;
+         add3(L.pos, d);
          acc_add(L.mom.x, -(dts * slope_p));
-         acc_add(L.pos.x, dr.x); acc_add(L.pos.y, dr.y); acc_add(L.pos.z, dr.z);
+         add3(L.pos, dr);
       }
       else {
-         add3(L.pos, dr - dts * slope);
+         d = dr - dts * slope;
+         add3(L.pos, d);
          acc_add(L.mom.x, -(dts * slope_p));
       }
    }
    if (sa != R(0)) L.amp += dts * sa * m_exp(L.wgt);
-   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S);
+   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
    L.steps++;
 }
 
@@ -1115,7 +1142,8 @@ __device__ __forceinline__ void parker_advance_gt(Lane<R, A>& L, BndView<R> bv, 
       return;
    }
    acc_add(L.pos.x, dr.x); acc_add(L.pos.y, dr.y); acc_add(L.pos.z, dr.z);
-   handle_boundaries<kParker, kLayoutAny>(L, bv, sp, s0, P, Pd, S);
+   L.clear = R(0);  // every boundary is evaluated
+   handle_boundaries<kParker, kLayoutAny>(L, bv, sp, s0, P, Pd, S, [] { return R(0); });
    L.steps++;
 }
 
@@ -1502,6 +1530,7 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
    }
    // RKSlopes: stage "is" (false: the trajectory ended or was discarded in it)
    auto stage = [&](int is) -> bool {
+      bool near = true;
       if constexpr (TAB::kGeneral) {
 #pragma unroll
          for (int il = 0; il < is; il++) {
@@ -1518,10 +1547,13 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
          const R dta = tab.template a<R>(is) * L.dt, ds = fwd ? dta : -dta;
 #pragma unroll
          for (int il = 0; il < is; il++) acc_add(L.t, ds);
-         add3(L.pos, ds * slp[is - 1]);
+         const V3<R> dp = ds * slp[is - 1];
+         add3(L.pos, dp);
          add3(L.mom, ds * slm[is - 1]);
+         // a stage point closer than the nearest boundary crosses none (0.81: the rounding of both sides)
+         near = !(norm2(dp) < R(0.81) * L.clear * L.clear && m_abs(L.clear) > Lim<R>::tiny);
       }
-      if (space_terminate<TT>(L, bv, sp, s0, P, Pd, S)) return false;
+      if (near && space_terminate<TT>(L, bv, sp, s0, P, Pd, S)) return false;
       V3<R> ms = lane_mom(L);
       if (!get_fields<BG>(P.bg, deriv_mode, (R)acc_val(L.t), val3<R>(L.pos), field_p<TT>(ms), traj_mask<TT>(), sp)) {
          L.status |= TRAJ_DISCARD;
@@ -1560,6 +1592,7 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
    }
    // RKStep
    if (fwd) acc_add(L.t, L.dt); else acc_add(L.t, -L.dt);
+   [[maybe_unused]] V3<R> d;
    if constexpr (kFP64) {
       [[maybe_unused]] V3<R> pos_lo = val3<R>(L.pos);
 #pragma unroll
@@ -1593,14 +1626,18 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
          dm = dm + w * slm[il];
       }
       R sdt = fwd ? L.dt : -L.dt;
-      add3(L.pos, sdt * dp);
+      d = sdt * dp;
+      add3(L.pos, d);
       add3(L.mom, sdt * dm);
    }
    if (gc_perp) {  // Advance: _pos += dr_perp after RKStep (src/trajectory_guiding_diff.cc:373)
       if constexpr (kFP64) { acc_add(L.pos.x, dr_perp.x); acc_add(L.pos.y, dr_perp.y); acc_add(L.pos.z, dr_perp.z); }
       else add3(L.pos, dr_perp);
    }
-   handle_boundaries<TT, kLayoutAny>(L, bv, sp, s0, P, Pd, S);
+   handle_boundaries<TT, kLayoutAny>(L, bv, sp, s0, P, Pd, S, [&] {
+      if constexpr (kFP64) return norm1(val3<R>(L.pos) - val3<R>(pos_loc));
+      else return norm1(d) + norm1(dr_perp);
+   });
    if (!(L.status & TRAJ_FINISH) && TT == kFocused) clamp_mu<A, R>(L.mom);
    L.steps++;
 }
@@ -1622,6 +1659,7 @@ __device__ __noinline__ void set_start(Lane<R, A>& L, BndView<R> bv, Start& s0, 
    L.dt = R(0);
    L.dt_adapt = R(0);
    L.src_del_old = R(0);
+   L.clear = R(0);
    InitRng rng{Pd.seed, L.traj_id, Pd.problem_id, L.attempt, 0u, 0u};
    double t = sample_time(rng, Pd, local);
    V3<double> pos = sample_pos(rng, Pd, local);
@@ -1705,7 +1743,7 @@ __device__ __forceinline__ void start_lane(Lane<R, A>& L, BndView<R> bv, Start& 
    L.t = n.t;
    L.pos.x = n.pos.x; L.pos.y = n.pos.y; L.pos.z = n.pos.z;
    L.mom.x = n.mom.x; L.mom.y = n.mom.y; L.mom.z = n.mom.z;
-   L.amp = n.amp; L.wgt = n.wgt; L.dt = n.dt; L.dt_adapt = n.dt_adapt; L.src_del_old = n.src_del_old;
+   L.amp = n.amp; L.wgt = n.wgt; L.dt = n.dt; L.dt_adapt = n.dt_adapt; L.src_del_old = n.src_del_old; L.clear = n.clear;
 }
 
 // ---- repacking the lanes of a block ----------------------------------------------------------
@@ -1738,7 +1776,7 @@ __device__ __forceinline__ void each_member(Lane<R, A>& L, F f)
    f(L.t);
    f(L.pos.x); f(L.pos.y); f(L.pos.z);
    f(L.mom.x); f(L.mom.y); f(L.mom.z);
-   f(L.amp); f(L.wgt); f(L.dt); f(L.dt_adapt); f(L.src_del_old);
+   f(L.amp); f(L.wgt); f(L.dt); f(L.dt_adapt); f(L.src_del_old); f(L.clear);
 }
 template <class R, class F>
 __device__ __forceinline__ void each_member(UniformStep<R>& h, F f)

@@ -2,6 +2,7 @@
 
 - Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
   1e140 takes the time-step bounds there (FP64 against the oracle).
+- Stage points told by their clearance from the boundaries, against the oracle's evaluation of each.
 - The FP32 kernels compiled for a boundary layout against the one that reads it from the descriptor.
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
@@ -16,7 +17,7 @@ import test_oracle_plugins as cases
 from spectrum_gb300 import capi, units
 from spectrum_gb300 import workloads as W
 from spectrum_gb300.datacontainer import DataContainer as DC
-from spectrum_gb300.plugins import DiffusionRigidityMagneticFieldPowerLaw
+from spectrum_gb300.plugins import BoundaryPlaneAbsorb, BoundaryPlaneReflect, DiffusionRigidityMagneticFieldPowerLaw
 from spectrum_gb300.simulation import open_problems, run_problems
 
 pytestmark = pytest.mark.gpu
@@ -122,8 +123,8 @@ def test_boundary_layout_kernels_equal_the_generic_one(built_lib, kind, n):
         pb = W.shock_acceleration(n_traj=n, width_frac=0.1, x_escape=-0.3, x_downstream=0.3, p_max=1.2)
     elif kind == "reflecting_planes_momentum_pass":
         pb = c._parker(n=n, bg=c._shock(), t_end=0.3,
-                       bnds=[(c.BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((0.2, 0, 0)).vec((1.0, 0, 0))),
-                             (c.BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((-0.2, 0, 0)).vec((-1.0, 0, 0))),
+                       bnds=[(BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((0.2, 0, 0)).vec((1.0, 0, 0))),
+                             (BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((-0.2, 0, 0)).vec((-1.0, 0, 0))),
                              (c.BoundaryMomentumPass(), c.B(DC(), -1, [0]).double(1.01))])
     else:
         pb = W.diffusion_uniform(n_traj=n, t_end=0.1)
@@ -138,3 +139,24 @@ def test_boundary_layout_kernels_equal_the_generic_one(built_lib, kind, n):
     for f in ("status", "steps", "t", "pos", "mom"):
         assert np.array_equal(out[0][1][f], out[1][1][f]), f
     assert np.array_equal(out[0][2][0], out[1][2][0])
+
+
+@pytest.mark.parametrize("offset", [0.0, 1.0e-3, 0.05, 0.9])
+@pytest.mark.parametrize("kind", ["sphere", "plane", "two_spheres_far_origin"])
+def test_stage_points_near_boundaries_match_oracle(built_lib, kind, offset):
+    """The clearance that stands in for the boundaries at stage points: Lorentz orbits (FP64) that start at various
+    distances from an absorbing boundary, on it among them, end at the same stage or step as in the oracle."""
+    c = cases
+    if kind == "sphere":
+        bnds = [(c.BoundarySphereAbsorb(), c.B(DC(), 1, [0]).vec((0, 0, 0)).double(1.0))]
+    elif kind == "plane":
+        bnds = [(BoundaryPlaneAbsorb(), c.B(DC(), 1, [0]).vec((1.0, 0, 0)).vec((1.0, 0, 0)))]
+    else:
+        bnds = [(c.BoundarySphereAbsorb(), c.B(DC(), 1, [0]).vec((1.0e6, 0, 0)).double(1.0e6 - 1.0)),
+                (c.BoundarySphereReflect(), c.B(DC(), -1, [-1]).vec((0, 0, 0)).double(3.0))]
+    bg = (c.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((0, 0, 0)).vec((0, 0.3, 1.0)).double(0.5))
+    pb = c._parker(n=48, traj=c.TRAJ_LORENTZ, diff=False, bg=bg, t_end=3.0, bnds=bnds,
+                   is_=(c.InitialSpaceFixed(), DC().vec((1.0 - offset, 0, 0))),
+                   im=(c.InitialMomentumShell(), DC().double(0.5)))
+    res = run_problems(pb, precision=capi.SPX_FP64, record=True)
+    ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
