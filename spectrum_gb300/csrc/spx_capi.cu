@@ -516,7 +516,7 @@ int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t tota
 // The FP64 pipe takes a warp instruction every 64 cycles of each scheduler, whatever its active lanes, so up to
 // one warp per scheduler is free: a launch that fits spreads over all schedulers (fewer trajectories a warp
 // diverge less), and where the kernel evaluates finite differences or pairs of normals its trajectories
-// get up to eight lanes each. Larger launches take one lane each and full warps; a caller's own launch shape
+// get up to eight lanes each, in the dipole four (a component each). Larger launches take one lane each and full warps; a caller's own launch shape
 // is kept as given.
 struct PlainShape {
    int64_t grid;
@@ -530,8 +530,9 @@ PlainShape plain_shape(const spx_ctx* c, int64_t total, int block, bool chosen_h
    if (chosen_here && c->precision == SPX_FP64 && total <= warps * 32) {
       const bool parker = c->traj == SPX_TRAJ_PARKER || c->traj == SPX_TRAJ_PARKER_SOURCE;
       const bool fd = c->deriv_mode == 0 && c->bg_kind == spx::kBgSolarWind;
-      if (parker || fd)
-         while (s.team < 8 && total * s.team * 2 <= warps * 32) s.team *= 2;
+      const bool split = c->bg_kind == spx::kBgDipole && (c->traj == SPX_TRAJ_LORENTZ || c->traj == SPX_TRAJ_GUIDING);
+      const int most = parker || fd ? 8 : (split ? 4 : 1);
+      while (s.team < most && total * s.team * 2 <= warps * 32) s.team *= 2;
       s.warp_lanes = s.team * (int)std::max<int64_t>(1, (total + warps - 1) / warps);
       s.block = 32;
    }

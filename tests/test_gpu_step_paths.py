@@ -67,7 +67,7 @@ def test_quotients_outside_the_fast_range(built_lib):
 
 
 @pytest.mark.parametrize("n", [1, 31, 700, 2433, 4865, 9729])
-@pytest.mark.parametrize("kind", ["modulation", "focused", "guiding"])
+@pytest.mark.parametrize("kind", ["modulation", "focused", "guiding", "lorentz"])
 def test_lane_teams_equal_single_lanes(built_lib, kind, n):
     """Small FP64 launches give a trajectory several lanes (eight up to 2,432 trajectories, four, two, then one) and
     spread over all schedulers; the launch shape given here has one lane each in full warps."""
@@ -75,8 +75,10 @@ def test_lane_teams_equal_single_lanes(built_lib, kind, n):
         pb = W.gcr_modulation(n_traj=n, energies_mev=[300.0], t_max_years=1.0e-4, pow_law_b=-1.0)[0]
     elif kind == "focused":
         pb = W.focused_transport(n_problems=1, n_traj=n, t_max_hours=0.002)[0]
-    else:
+    elif kind == "guiding":
         pb = W.guiding_dipole(n_traj=n, t_end_s=0.1)
+    else:
+        pb = W.dipole_orbits(n_traj=n, t_end=0.01 / units.unit_time)
     a = run_problems(pb, precision=capi.SPX_FP64, record=True)
     b = run_problems(pb, precision=capi.SPX_FP64, record=True, tuning=capi.Tuning(128, 0, 0, 0))
     assert a.stats.trajectories == b.stats.trajectories == n and a.stats.steps == b.stats.steps > n
