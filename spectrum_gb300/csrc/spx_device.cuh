@@ -100,6 +100,14 @@ template <> struct Divisor<double> {
 };
 template <class R> __device__ __forceinline__ R quot(R x, R y) { return Divisor<R>(y)(x); }
 
+// x is finite and not zero (in double by integer tests, which leave the FP64 pipe alone)
+__device__ __forceinline__ bool finite_nonzero(float x) { return isfinite(x) && x != 0.0f; }
+__device__ __forceinline__ bool finite_nonzero(double x)
+{
+   const int hi = __double2hiint(x), lo = __double2loint(x);
+   return (((unsigned)hi >> 20) & 0x7ffu) != 0x7ffu && ((hi << 1) | lo) != 0;
+}
+
 // ---- 3-vectors ------------------------------------------------------------------------------
 template <class R>
 struct V3 {

@@ -604,19 +604,42 @@ __device__ __forceinline__ bool space_terminate(Lane<R, A>& L, BndView<R> bv, co
    return false;
 }
 
-// TimeBoundaryProximityCheck (src/trajectory_base.cc:151-179)
+// What the step's checks take from dmax: "no time boundary ahead" and the least step towards one
+// (TimeBoundaryProximityCheck), and the step too small to go on with (Integrate). Evaluated where they are read, or
+// held (StepLimits) where dmax is a constant of the trajectory.
 template <class R>
-__device__ __forceinline__ R time_proximity(R dt, R dmax, BndView<R> bv, int nbt, bool fwd)
+struct DmaxLimits {
+   R dmax;
+   __device__ __forceinline__ R none() const { return over_c(Lim<R>::large * dmax); }
+   __device__ __forceinline__ R least() const { return over_c(Lim<R>::small * dmax); }
+   __device__ __forceinline__ R error() const { return over_c(Lim<R>::tiny * dmax); }
+};
+template <class R>
+struct StepLimits {
+   R none_, least_, error_;
+   __device__ __forceinline__ R none() const { return none_; }
+   __device__ __forceinline__ R least() const { return least_; }
+   __device__ __forceinline__ R error() const { return error_; }
+};
+
+// TimeBoundaryProximityCheck (src/trajectory_base.cc:151-179)
+template <class R, class LIM>
+__device__ __forceinline__ R time_proximity(R dt, const LIM& lim, BndView<R> bv, int nbt, bool fwd)
 {
-   R dn = over_c(fwd ? -Lim<R>::large * dmax : Lim<R>::large * dmax);
+   R dn = fwd ? -lim.none() : lim.none();
    for (int b = 0; b < nbt; b++) {
       R delta = bv.ld(b).delta;
       if (fwd) { if (delta <= R(0) && delta > dn) dn = delta; }
       else { if (delta >= R(0) && delta < dn) dn = delta; }
    }
-   if (fwd) { if (dt >= -dn) dt = m_max(-(R(1) + Lim<R>::little) * dn, over_c(Lim<R>::small * dmax)); }
-   else { if (dt >= dn) dt = m_max((R(1) + Lim<R>::little) * dn, over_c(Lim<R>::small * dmax)); }
+   if (fwd) { if (dt >= -dn) dt = m_max(-(R(1) + Lim<R>::little) * dn, lim.least()); }
+   else { if (dt >= dn) dt = m_max((R(1) + Lim<R>::little) * dn, lim.least()); }
    return dt;
+}
+template <class R>
+__device__ __forceinline__ R time_proximity(R dt, R dmax, BndView<R> bv, int nbt, bool fwd)
+{
+   return time_proximity(dt, DmaxLimits<R>{dmax}, bv, nbt, fwd);
 }
 
 // UpdateBmagExtrema (src/trajectory_base.cc:586-592) of the previous step: the reference folds in the
@@ -639,10 +662,10 @@ __device__ __forceinline__ void track_bmag(Start& s0, const RunConfig& cfg, cons
 // dmax of the point where that step ended. That point is where this step starts, so the dmax of
 // this step's field evaluation is the same number the reference compares with; a failed check
 // discards the attempt before anything else of this step happens.
-template <class R, class A>
-__device__ __forceinline__ bool prev_step_ok(Lane<R, A>& L, R dmax)
+template <class R, class A, class LIM>
+__device__ __forceinline__ bool prev_step_ok(Lane<R, A>& L, const LIM& lim)
 {
-   if (L.steps > 0 && !(L.dt >= over_c(Lim<R>::tiny * dmax))) {
+   if (L.steps > 0 && !(L.dt >= lim.error())) {
       L.status |= TRAJ_DISCARD;
       return false;
    }
@@ -755,7 +778,16 @@ __device__ __forceinline__ void step_normals(uint4 b, float n[4]) { normals4<flo
 __device__ __forceinline__ void step_normals(uint4 b, double n[4])
 {
    const Team tm = my_team();
-   if (tm.size == 1) { normals4<double>(b, n); return; }
+   if (tm.size == 1) {
+      // the fourth normal is not used: cospi, which equals sincospi's cosine for every one of the 2^32 deviates
+      const double r0 = m_sqrt(-2.0 * m_log(u01d(b.x))), r1 = m_sqrt(-2.0 * m_log(u01d(b.z)));
+      double s0, c0;
+      sincos_2pi(u01d(b.y), &s0, &c0);
+      n[0] = r0 * c0;
+      n[1] = r0 * s0;
+      n[2] = r1 * cospi(2.0 * u01d(b.w));
+      return;
+   }
    const bool odd = tm.rank & 1;
    const double r = m_sqrt(-2.0 * m_log(u01d(odd ? b.z : b.x)));
    double s, c;
@@ -779,6 +811,7 @@ struct UniformStep {
    bool valid;
    V3<R> slope, fa[3];
    R slope_p, sperp, spara, dtp, dmax, Bmag, divU;
+   StepLimits<R> lim;
 };
 
 // The diffusion classes whose coefficients do not read the position (kappa_pp), so that in a uniform field
@@ -822,6 +855,8 @@ __device__ __noinline__ void uniform_step(const ProblemDescT<R>& P, int deriv_mo
    h.fa[0] = second_unit(sp.bhat);
    h.fa[1] = cross(h.fa[2], h.fa[0]);
    h.dmax = sp.dmax;
+   const DmaxLimits<R> lim{sp.dmax};
+   h.lim = {lim.none(), lim.least(), lim.error()};
    h.Bmag = sp.Bmag;
    h.valid = true;
 }
@@ -832,10 +867,10 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
                                                        const ProblemDescT<R>& P, const ProblemDesc& Pd, bool fwd, const Sinks& S)
 {
    constexpr bool kFP64 = sizeof(R) == sizeof(double);
-   if (!prev_step_ok(L, h.dmax)) return;
+   if (!prev_step_ok(L, h.lim)) return;
    // |B| is the first point's everywhere: its extrema need no fold
    const R sa = P.src.kind ? parker_source(L, P, (R)acc_val(L.mom.x), val3<R>(L.pos)) : R(0);
-   L.dt = time_proximity(h.dtp, h.dmax, bv, n_time_bnd<BL>(P), fwd);
+   L.dt = time_proximity(h.dtp, h.lim, bv, n_time_bnd<BL>(P), fwd);
    R n[4];
    step_normals(rng_block(P.seed, L.steps, L.traj_id, P.problem_id, kRngStep, L.attempt), n);
    R sdt = m_sqrt(L.dt);
@@ -897,7 +932,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    SD<R> sp;
    const unsigned mask = traj_mask<kParker>() | (kappa_grad_is_analytic(P.df, DK) ? kDerivedOnly : 0u);
    if (!get_fields<BG>(P.bg, deriv_mode, t, pos, p, mask, sp)) { L.status |= TRAJ_DISCARD; return; }
-   if (!prev_step_ok(L, sp.dmax)) return;
+   if (!prev_step_ok(L, DmaxLimits<R>{sp.dmax})) return;
    track_bmag(s0, cfg, sp);
    R vmag = vel_of(p);
    // DiffusionCoeff (src/trajectory_parker.cc:83-153)
@@ -1071,7 +1106,7 @@ __device__ __forceinline__ void parker_advance_gt(Lane<R, A>& L, BndView<R> bv, 
    const R p = (R)acc_val(L.mom.x);
    SD<R> sp;
    if (!get_fields<BG>(P.bg, deriv_mode, (R)acc_val(L.t), pos, p, mask, sp)) { L.status |= TRAJ_DISCARD; return; }
-   if (!prev_step_ok(L, sp.dmax)) return;
+   if (!prev_step_ok(L, DmaxLimits<R>{sp.dmax})) return;
    track_bmag(s0, cfg, sp);
    V3<R> slp[SPX_RK_MAX_STAGES];
    R slm[SPX_RK_MAX_STAGES], sla[SPX_RK_MAX_STAGES];
@@ -1380,7 +1415,7 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
    if (gc_perp) zero(sp.gradU);
    R d_perp = R(0);
    V3<R> fa[3];
-   if (!prev_step_ok(L, sp.dmax)) return;
+   if (!prev_step_ok(L, DmaxLimits<R>{sp.dmax})) return;
    track_bmag(s0, cfg, sp);
    if (!split) vel = vel_load<TT>(mom);
    V3<R> drift = mk(R(0), R(0), R(0));
@@ -1876,6 +1911,7 @@ __device__ __forceinline__ void each_member(UniformStep<R>& h, F f)
    f(h.slope.x); f(h.slope.y); f(h.slope.z);
    for (int k = 0; k < 3; k++) { f(h.fa[k].x); f(h.fa[k].y); f(h.fa[k].z); }
    f(h.slope_p); f(h.sperp); f(h.spara); f(h.dtp); f(h.dmax); f(h.Bmag); f(h.divU);
+   f(h.lim.none_); f(h.lim.least_); f(h.lim.error_);
 }
 
 // Moves the words and boundary states of the block's active lanes to its first threads, in order; every
@@ -2063,7 +2099,7 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
                rk_advance<TT, BG, R, A, FixedRk<4>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<4>{});
             else rk_advance<TT, BG, R, A, FixedRk<1>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<1>{});
             // Integrate's safety limits (src/trajectory_base.cc:964-992)
-            if (L.steps > kMaxTrajSteps || !isfinite(L.dt) || L.dt == R(0)) L.status |= TRAJ_DISCARD;
+            if (L.steps > kMaxTrajSteps || !finite_nonzero(L.dt)) L.status |= TRAJ_DISCARD;
             done = (L.status & TRAJ_FINISH) && !(L.status & TRAJ_DISCARD);
             // timing samples of the autotuner stop every trajectory after a fixed number of steps
             if (cfg.step_cap && L.steps >= cfg.step_cap && !done) {
