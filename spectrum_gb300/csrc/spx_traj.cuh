@@ -1305,8 +1305,24 @@ __device__ __forceinline__ void rk_slopes(const SD<R>& s, V3<R> mom, V3<R> vel, 
    }
 }
 
+// A vector's components over the first three lanes of each four of a team (the fourth repeats the first).
+struct SplitVector {
+   Team tm;
+   int c;
+   __device__ __forceinline__ SplitVector() : tm(my_team()) { c = (tm.rank & 3) == 3 ? 0 : tm.rank & 3; }
+   __device__ __forceinline__ double own(V3<double> v) const { return c == 0 ? v.x : (c == 1 ? v.y : v.z); }
+   __device__ __forceinline__ V3<double> all(double v) const { return mk(tm.from(v, 0), tm.from(v, 1), tm.from(v, 2)); }
+   __device__ __forceinline__ double sum(double p) const { const V3<double> q = all(p); return q.x + q.y + q.z; }
+   __device__ __forceinline__ double cross(V3<double> a, V3<double> b) const
+   {
+      const double a1 = c == 0 ? a.y : (c == 1 ? a.z : a.x), a2 = c == 0 ? a.z : (c == 1 ? a.x : a.y);
+      const double b1 = c == 0 ? b.y : (c == 1 ? b.z : b.x), b2 = c == 0 ? b.z : (c == 1 ? b.x : b.y);
+      return a1 * b2 - a2 * b1;
+   }
+};
+
 // Fields, velocity and slopes at one point of the dipole by a team of four lanes or more (FP64): lane c has
-// component c of every vector (the fourth repeats the first), so a vector operation is one FP64 instruction
+// component c of every vector (SplitVector), so a vector operation is one FP64 instruction
 // instead of three and the lanes have a row of grad B each; sums of products are gathered and added by every lane
 // in the order that one lane adds them. The operations are those of get_fields, vel_cart and rk_slopes
 // (guiding_drift for TrajectoryGuiding), with what vanishes in the dipole left out: E, and curl B, whose
@@ -1317,56 +1333,47 @@ __device__ __noinline__ bool dipole_slopes_split(const BgParams& g, V3<double> p
                                                  V3<double>& sp, V3<double>& sm)
 {
    static_assert(TT == kLorentz || TT == kGuiding, "types with a split dipole point");
-   const Team tm = my_team();
-   const int c = (tm.rank & 3) == 3 ? 0 : tm.rank & 3;
-   auto own = [&](V3<double> v) { return c == 0 ? v.x : (c == 1 ? v.y : v.z); };
-   auto all = [&](double v) { return mk(tm.from(v, 0), tm.from(v, 1), tm.from(v, 2)); };
-   auto sum = [&](double p) { const V3<double> q = all(p); return q.x + q.y + q.z; };
-   auto cross_own = [&](V3<double> a, V3<double> b) {
-      const double a1 = c == 0 ? a.y : (c == 1 ? a.z : a.x), a2 = c == 0 ? a.z : (c == 1 ? a.x : a.y);
-      const double b1 = c == 0 ? b.y : (c == 1 ? b.z : b.x), b2 = c == 0 ? b.z : (c == 1 ? b.x : b.y);
-      return a1 * b2 - a2 * b1;
-   };
-   const double m1 = own(mom), m = m_sqrt(sum(m1 * m1));
-   vel = all((vel_of(m) / m) * m1);
+   const SplitVector l;
+   const double m1 = l.own(mom), m = m_sqrt(l.sum(m1 * m1));
+   vel = l.all((vel_of(m) / m) * m1);
    const V3<double> M = ld3(g.M);
-   const double x = own(pos) - own(ld3(g.r0)), Mc = own(M);
-   const double r = m_sqrt(sum(x * x)), r2 = r * r, r5 = r2 * r * r2;
+   const double x = l.own(pos) - l.own(ld3(g.r0)), Mc = l.own(M);
+   const double r = m_sqrt(l.sum(x * x)), r2 = r * r, r5 = r2 * r * r2;
    s.dmax = m_min(g.dmax_fraction * r, g.dmax0);
-   const double xm = sum(x * Mc);
+   const double xm = l.sum(x * Mc);
    const Divisor<double> over5(r5);
    const double b = over5(3.0 * xm * x - r2 * Mc);
-   s.B = all(b);
-   s.Bmag = norm(s.B);
+   s.B = l.all(b);
+   s.Bmag = m_sqrt(l.sum(b * b));
    if (!(s.Bmag >= Lim<double>::tiny)) return false;
    const Divisor<double> over_B(s.Bmag);
    const double bh = over_B(b);
-   s.bhat = all(bh);
+   s.bhat = l.all(bh);
    s.E = mk(0.0, 0.0, 0.0);
    s.region = mk(1.0, 1.0, 1.0);
    s.divU = 0.0;
    if constexpr (TT == kLorentz) {
       sp = vel;
-      sm = all(0.0 + over_c(cross_own(vel, s.B)));
+      sm = l.all(0.0 + over_c(l.cross(vel, s.B)));
    }
    else {
       const double cl = c_code<double>();
-      const V3<double> xs = all(x);
+      const V3<double> xs = l.all(x);
       const Divisor<double> over2(r2);
       double row[3];
 #pragma unroll
       for (int k = 0; k < 3; k++)
-         row[k] = over5(3.0 * (Mc * xs[k] + x * M[k] + xm * ((c == k ? 1.0 : 0.0) - over2(5.0 * (x * xs[k])))));
+         row[k] = over5(3.0 * (Mc * xs[k] + x * M[k] + xm * ((l.c == k ? 1.0 : 0.0) - over2(5.0 * (x * xs[k])))));
       const double gb = row[0] * s.bhat.x + row[1] * s.bhat.y + row[2] * s.bhat.z;
       const double rL = over_B(mom.x * cl), rR = over_B(mom.z * cl);
-      const double curl = over_B(0.0 - cross_own(all(gb), s.bhat));
+      const double curl = over_B(0.0 - l.cross(l.all(gb), s.bhat));
       const double e = 0.0 - over_2c(rL * vel.x * gb);
       const double bs = b + rR * s.Bmag * curl;
-      const double bsb = sum(bs * bh);
+      const double bsb = l.sum(bs * bh);
       const Divisor<double> over_bsb(bsb);
-      const double d = over_bsb(vel.z * bs + cl * cross_own(all(e), s.bhat));
-      sp = all(d);
-      sm = mk(over_B(0.5 * mom.x) * (0.0 + sum(d * gb)), 0.0, over_bsb(sum(e * bs)));
+      const double d = over_bsb(vel.z * bs + cl * l.cross(l.all(e), s.bhat));
+      sp = l.all(d);
+      sm = mk(over_B(0.5 * mom.x) * (0.0 + l.sum(d * gb)), 0.0, over_bsb(l.sum(e * bs)));
    }
    return true;
 }
@@ -1658,11 +1665,27 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
          const R dta = tab.template a<R>(is) * L.dt, ds = fwd ? dta : -dta;
 #pragma unroll
          for (int il = 0; il < is; il++) acc_add(L.t, ds);
-         const V3<R> dp = ds * slp[is - 1];
-         add3(L.pos, dp);
-         add3(L.mom, ds * slm[is - 1]);
+         R dist2;
+         bool added = false;
+         if constexpr (kSplit) {
+            if (split) {
+               const SplitVector l;
+               const double d = ds * l.own(slp[is - 1]);
+               dist2 = l.sum(d * d);
+               const V3<R> p = l.all(l.own(val3<R>(L.pos)) + d), m = l.all(l.own(lane_mom(L)) + ds * l.own(slm[is - 1]));
+               L.pos.x = p.x; L.pos.y = p.y; L.pos.z = p.z;
+               L.mom.x = m.x; L.mom.y = m.y; L.mom.z = m.z;
+               added = true;
+            }
+         }
+         if (!added) {
+            const V3<R> dp = ds * slp[is - 1];
+            add3(L.pos, dp);
+            add3(L.mom, ds * slm[is - 1]);
+            dist2 = norm2(dp);
+         }
          // a stage point closer than the nearest boundary crosses none (0.81: the rounding of both sides)
-         near = !(norm2(dp) < R(0.81) * L.clear * L.clear && m_abs(L.clear) > Lim<R>::tiny);
+         near = !(dist2 < R(0.81) * L.clear * L.clear && m_abs(L.clear) > Lim<R>::tiny);
       }
       if (near && space_terminate<TT>(L, bv, sp, s0, P, Pd, S)) return false;
       V3<R> ms = lane_mom(L);
@@ -1719,6 +1742,24 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
    [[maybe_unused]] V3<R> d;
    if constexpr (kFP64) {
       [[maybe_unused]] V3<R> pos_lo = val3<R>(L.pos);
+      bool added = false;
+      if constexpr (kSplit && !TAB::kGeneral) {
+         if (split) {
+            const SplitVector l;
+            double p = l.own(val3<R>(L.pos)), m = l.own(lane_mom(L));
+#pragma unroll
+            for (int il = 0; il < TAB::kMax; il++) {
+               const double wdt = L.dt * tab.template v<R>(il), w = fwd ? wdt : -wdt;
+               p += w * l.own(slp[il]);
+               m += w * l.own(slm[il]);
+            }
+            const V3<R> ps = l.all(p), ms = l.all(m);
+            L.pos.x = ps.x; L.pos.y = ps.y; L.pos.z = ps.z;
+            L.mom.x = ms.x; L.mom.y = ms.y; L.mom.z = ms.z;
+            added = true;
+         }
+      }
+      if (!added)
 #pragma unroll
       for (int il = 0; il < (TAB::kGeneral ? tab.stages() : TAB::kMax); il++) {
          R w = L.dt * tab.template v<R>(il);
