@@ -956,22 +956,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    V3<R> slope = fwd ? sp.U + divK : sp.U - divK;
    R divU = sd_divU(sp);
    R slope_p = -p * divU / R(3);
-   R sa = R(0);
-   if (P.src.kind == 1) sa = P.src.rate;  // SourceConstant: S0 every step (src/source_other.cc:41-59)
-   else if (P.src.kind >= 2) {
-      // TrajectoryParkerSource::Slopes / SourceMomentumInjection::EvaluateSource
-      // (src/trajectory_parker_source.cc:58-66, src/source_other.cc:113-119); dt is the previous step's.
-      // SourceSphericalShockInjection (:166-177) injects only inside the shell r_sh <= |r - r0| <= r_sh + w_sh.
-      R del = p - P.src.p_inj;
-      if (del * L.src_del_old < R(0)) {
-         if (P.src.kind == 2) sa = P.src.rate / L.dt;
-         else {
-            R r = norm(pos - ld3(P.src.r0));
-            if (P.src.r_sh <= r && r <= P.src.r_sh + P.src.w_sh) sa = P.src.rate / L.dt;
-         }
-      }
-      L.src_del_old = del;
-   }
+   const R sa = P.src.kind ? parker_source(L, P, p, pos) : R(0);
    // PhysicalStep (src/trajectory_parker.cc:212-221)
    R dtp;
    // on a grid the wide and deep builds would fuse different products of the sum: it is fixed here
@@ -2139,6 +2124,11 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             else if (cfg.rk == 25)
                rk_advance<TT, BG, R, A, FixedRk<4>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<4>{});
             else rk_advance<TT, BG, R, A, FixedRk<1>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<1>{});
+            // one test for all that can follow a step (Parker; it made the longer Runge-Kutta steps no faster)
+            if constexpr (TT == kParker && !GT) {
+               const bool limits = L.steps > kMaxTrajSteps || !finite_nonzero(L.dt);
+               if (__builtin_expect(!(limits || L.status || cfg.step_cap), 1)) continue;
+            }
             // Integrate's safety limits (src/trajectory_base.cc:964-992)
             if (L.steps > kMaxTrajSteps || !finite_nonzero(L.dt)) L.status |= TRAJ_DISCARD;
             done = (L.status & TRAJ_FINISH) && !(L.status & TRAJ_DISCARD);
