@@ -481,7 +481,8 @@ int64_t deep_lanes_limit(const spx_ctx* c)
 // The launch shape of a run: the caller's, else the one spx_autotune chose, else the defaults (the
 // FP64 drop-in keeps one thread per trajectory; the FP32 stepper takes the persistent queue in
 // blocks of 64 refilled every 8 steps, the shape that measured fastest on the modulation batch, or up to
-// deep_lanes_limit the kernels' deep build in blocks of 128, whose warps it repacks).
+// deep_lanes_limit the kernels' deep build in blocks of 128, whose warps it repacks; the guiding centres' kernels
+// repack in their one build).
 // Unset fields are completed and checked; blocks per SM is capped by the kernel's occupancy for
 // "slots" boundary states per lane. Shared by spx_run and spx_run_static.
 int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t total, spx_tuning& tu, bool& deep)
@@ -493,7 +494,8 @@ int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t tota
    else {
       tu.schedule = c->precision == SPX_MIXED ? 1 : 0;
       if (tu.schedule) {
-         tu.block_size = 64;
+         const bool guiding = c->traj >= SPX_TRAJ_GUIDING && c->traj <= SPX_TRAJ_GUIDING_DIFF_SCATT;
+         tu.block_size = guiding ? 128 : 64;  // the guiding centres' kernels repack their blocks
          tu.steps_per_sync = 8;
          const int occ = occupancy(c, 128, slots, true);
          if (occ > 0 && total <= deep_lanes_limit(c) * c->sm_count * 128 * occ) {

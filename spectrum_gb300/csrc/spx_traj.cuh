@@ -1992,10 +1992,13 @@ constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
 // kDkNoDiffusion: the guiding-centre kernels for TrajectoryGuiding proper (no scattering, no perpendicular step).
 // BL: the boundary layout (BndLayout) the Parker step is compiled for; kLayoutAny reads it from the
 // descriptor.
-// MB: resident blocks of 128 per SM (above); the wide FP32 build does not repack its lanes.
+// MB: resident blocks of 128 per SM (above); the wide FP32 build does not repack its lanes, but for the guiding
+// centres, which have no other: orbits' step counts differ by a factor of five, and repacking took 1e5 of them from
+// 32.3 to 26.6 ms (2e5 27.2 -> 25.0, 1e3 7.56 -> 7.29; focused transport lost 4% below 1e5 trajectories).
 // Steps between two barriers of a draining block: few enough that a warp emptied early is soon given up,
-// enough that waiting for the slowest of the block's warps costs little.
-constexpr int kDrainSteps = 32;
+// enough that waiting for the slowest of the block's warps costs little (32 to 128 are within 2% of each other;
+// grid transport 366 ms at 32, 355 at 64).
+constexpr int kDrainSteps = 64;
 
 template <int TT, int BG, class R, int DM, bool GT, int DK, int BL, int MB>
 __global__ void __launch_bounds__(128, MB)
@@ -2032,7 +2035,7 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
    }
    // The plain grid drains from the start. The queue's lanes refill until a warp of the block finds it dry;
    // then the block's warps go on together: K steps, a barrier, and a repacking where it empties a warp.
-   constexpr bool kRepack = MB != kWideBlocksF32;
+   constexpr bool kRepack = MB != kWideBlocksF32 || TT == kGuiding;
    __shared__ unsigned long long s_buf[kRepack ? 128 : 1];
    __shared__ volatile int s_dry;
    if constexpr (kRepack) {

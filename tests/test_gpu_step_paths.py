@@ -162,3 +162,17 @@ def test_stage_points_near_boundaries_match_oracle(built_lib, kind, offset):
                    im=(c.InitialMomentumShell(), DC().double(0.5)))
     res = run_problems(pb, precision=capi.SPX_FP64, record=True)
     ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
+
+
+@pytest.mark.parametrize("n", [1, 129, 4097, 120_001])
+def test_guiding_repacking_keeps_the_orbits(built_lib, n):
+    """FP32 guiding centres in blocks of 128, whose warps are repacked as orbits end, against blocks of one warp, which
+    have nothing to repack: mirror-point events and final states, bit for bit."""
+    pb = W.guiding_dipole(n_traj=n, t_end_s=0.5)
+    a = run_problems(pb, precision=capi.SPX_MIXED, record=True)
+    b = run_problems(pb, precision=capi.SPX_MIXED, record=True, tuning=capi.Tuning(32, 0, 8, 1))
+    assert a.stats.tuning.block_size == 128 and a.stats.steps == b.stats.steps and a.stats.events == b.stats.events
+    for f in ("attempts", "status", "steps", "t", "pos", "mom", "pos0", "mom0"):
+        assert np.array_equal(a.records[0][f], b.records[0][f]), f
+    for (ca, _, na), (cb, _, nb) in zip(a.distros[0], b.distros[0]):
+        assert na == nb and np.array_equal(ca, cb)
