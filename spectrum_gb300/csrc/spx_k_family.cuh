@@ -2,7 +2,7 @@
 // trajectory family, arithmetic, field-derivative method and table kind (Euler and the classic RK4
 // with unrolled constants, or any Butcher table from constant memory), and for the FP32 Parker kernels
 // a diffusion class and boundary layout fixed at compile time, switching over the background classes.
-// Each spx_k_*.cu instantiates it once, so the 24 kernel sets compile in parallel.
+// Each spx_k_*.cu instantiates it once, so the kernel sets compile in parallel.
 #pragma once
 
 #include "spx_launch.hh"
@@ -19,9 +19,11 @@ struct FamilyTU {
    template <int BG>
    static constexpr bool kBuilt = !(TT == kGuiding && (BG == kBgShock || BG == kBgSmoothShock));
 
-   // Parker and Lorentz in FP32 have the deep build too
+   // Lorentz, and Parker with the diffusion class fixed, have the deep FP32 build too. (The generic Parker kernel has not:
+   // at three blocks the compiler fuses other products of its run-time dispatch in the solar wind, and its trajectories
+   // would no longer be those of the kernels compiled for a class.)
    static constexpr int kBlocks = sizeof(R) == 4 ? kWideBlocksF32 : kBlocksF64;
-   static constexpr bool kHasDeep = sizeof(R) == 4 && (TT == kParker || TT == kLorentz);
+   static constexpr bool kHasDeep = sizeof(R) == 4 && ((TT == kParker && DK >= 0) || TT == kLorentz);
 
    template <int BG, int MB>
    static cudaError_t go_build(const LaunchArgs& a)
