@@ -529,11 +529,12 @@ __device__ __forceinline__ int n_space_bnd(const ProblemDescT<R>& P)
 template <int BL, class R>
 __device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL == kLayoutAny ? P.nbm : (BL == kLayoutPlanes ? 1 : 0); }
 
-// moved() is no less than the distance moved since the last call: while the clearance lasts no spatial
+// CL: moved() is no less than the distance moved since the last call: while the clearance lasts no spatial
 // boundary can have been crossed, and none is evaluated (a state's delta_old is then an older one of the same sign;
 // of an absorbing or passing boundary only the sign is read). One GB300: focused transport 326 -> 286 ms, shock
-// acceleration 286 -> 268 ms, modulation 245 -> 238 ms.
-template <int TT, int BL, class R, class A, class F>
+// acceleration 286 -> 268 ms, modulation 245 -> 238 ms. Not in the wide FP32 Parker kernels, whose warps wait for issue
+// slots and registers, not for the evaluation (modulation with every lane busy 4.84e10 -> 4.61e10 steps/s with it).
+template <int TT, int BL, bool CL, class R, class A, class F>
 __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, const SD<R>& sp, const Start& s0,
                                                   const ProblemDescT<R>& P, const ProblemDesc& Pd, const Sinks& S, F moved)
 {
@@ -548,7 +549,17 @@ __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, 
       else b.delta_old = b.delta;
       bv.st(j, b);
    }
-   if (nbs > 0) {
+   if constexpr (!CL) {
+      for (int i = 0; i < nbs; i++) {
+         const int j = nbt + i;
+         BndState<R> b = bv.ld(j);
+         compute_bnd<1, BL>(P.bs[i], b, L.t, pos, mom, sp.bhat, sp.region, TT);
+         if (b.crossed) crossed |= 1u << j;
+         else b.delta_old = b.delta;
+         bv.st(j, b);
+      }
+   }
+   else if (nbs > 0) {
       L.clear = sub_down(L.clear, moved() * R(1.0001));
       if (!(L.clear > Lim<R>::tiny)) {
          R clear = Lim<R>::large;
@@ -862,7 +873,7 @@ __device__ __noinline__ void uniform_step(const ProblemDescT<R>& P, int deriv_mo
 }
 
 // One step from held coefficients: parker_advance with the evaluations at the start point left out.
-template <int BL, class R, class A>
+template <int BL, bool CL, class R, class A>
 __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R> bv, Start& s0, const UniformStep<R>& h,
                                                        const ProblemDescT<R>& P, const ProblemDesc& Pd, bool fwd, const Sinks& S)
 {
@@ -896,12 +907,12 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    sp.region = mk(R(1), R(1), R(1));
    sp.Bmag = h.Bmag;
    sp.divU = h.divU;
-   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
+   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
    L.steps++;
 }
 
 // h: the held coefficients of a uniform field (BackgroundUniform only).
-template <int BG, int DK, int BL, class R, class A>
+template <int BG, int DK, int BL, bool CL, class R, class A>
 __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Start& s0, UniformStep<R>& h,
                                                const ProblemDescT<R>& P, const ProblemDesc& Pd, const RunConfig& cfg,
                                                const Sinks& S)
@@ -918,7 +929,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
          h = u;
       }
       if (h.valid) {
-         parker_uniform_advance<BL>(L, bv, s0, h, P, Pd, fwd, S);
+         parker_uniform_advance<BL, CL>(L, bv, s0, h, P, Pd, fwd, S);
          return;
       }
       if constexpr (DK >= 0) {  // a position-free class (every class with kernels of its own): a field error
@@ -1016,7 +1027,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
       }
    }
    if (sa != R(0)) L.amp += dts * sa * m_exp(L.wgt);
-   handle_boundaries<kParker, BL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
+   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
    L.steps++;
 }
 
@@ -1163,7 +1174,7 @@ __device__ __forceinline__ void parker_advance_gt(Lane<R, A>& L, BndView<R> bv, 
    }
    acc_add(L.pos.x, dr.x); acc_add(L.pos.y, dr.y); acc_add(L.pos.z, dr.z);
    L.clear = R(0);  // every boundary is evaluated
-   handle_boundaries<kParker, kLayoutAny>(L, bv, sp, s0, P, Pd, S, [] { return R(0); });
+   handle_boundaries<kParker, kLayoutAny, true>(L, bv, sp, s0, P, Pd, S, [] { return R(0); });
    L.steps++;
 }
 
@@ -1784,7 +1795,7 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
       if constexpr (kFP64) { acc_add(L.pos.x, dr_perp.x); acc_add(L.pos.y, dr_perp.y); acc_add(L.pos.z, dr_perp.z); }
       else add3(L.pos, dr_perp);
    }
-   handle_boundaries<TT, kLayoutAny>(L, bv, sp, s0, P, Pd, S, [&] {
+   handle_boundaries<TT, kLayoutAny, true>(L, bv, sp, s0, P, Pd, S, [&] {
       if constexpr (kFP64) return norm1(val3<R>(L.pos) - val3<R>(pos_loc));
       else return norm1(d) + norm1(dr_perp);
    });
@@ -2036,6 +2047,8 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
    // The plain grid drains from the start. The queue's lanes refill until a warp of the block finds it dry;
    // then the block's warps go on together: K steps, a barrier, and a repacking where it empties a warp.
    constexpr bool kRepack = MB != kWideBlocksF32 || TT == kGuiding;
+   // what shortens a lone warp's step at the cost of registers: not in the wide build of the Parker kernels
+   constexpr bool kShortChain = MB != kWideBlocksF32;
    __shared__ unsigned long long s_buf[kRepack ? 128 : 1];
    __shared__ volatile int s_dry;
    if constexpr (kRepack) {
@@ -2123,12 +2136,13 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
                if (TT == kParker) parker_advance_gt<BG>(L, bv, s0, Pp, Pd[L.prob], cfg, S, tab);
                else rk_advance<TT, BG, R, A>(L, bv, s0, Pp, Pd[L.prob], cfg, S, tab);
             }
-            else if (TT == kParker) parker_advance<BG, DK, BL>(L, bv, s0, held, Pp, Pd[L.prob], cfg, S);
+            else if (TT == kParker) parker_advance<BG, DK, BL, kShortChain>(L, bv, s0, held, Pp, Pd[L.prob], cfg, S);
             else if (cfg.rk == 25)
                rk_advance<TT, BG, R, A, FixedRk<4>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<4>{});
             else rk_advance<TT, BG, R, A, FixedRk<1>, DK == kDkNoDiffusion>(L, bv, s0, Pp, Pd[L.prob], cfg, S, FixedRk<1>{});
-            // one test for all that can follow a step (Parker; it made the longer Runge-Kutta steps no faster)
-            if constexpr (TT == kParker && !GT) {
+            // one test for all that can follow a step (Parker; it made the longer Runge-Kutta steps no faster, and the wide
+            // build slower: 4.84e10 -> 4.76e10 steps/s)
+            if constexpr (TT == kParker && !GT && kShortChain) {
                const bool limits = L.steps > kMaxTrajSteps || !finite_nonzero(L.dt);
                if (__builtin_expect(!(limits || L.status || cfg.step_cap), 1)) continue;
             }
