@@ -5,6 +5,7 @@
 - Stage points told by their clearance from the boundaries, against the oracle's evaluation of each.
 - The FP32 kernels compiled for a boundary layout against the one that reads it from the descriptor.
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
+- The initial momentum, of whose two samples the first is only counted where nothing reads it, against the oracle.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
   and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
@@ -17,7 +18,8 @@ import test_oracle_plugins as cases
 from spectrum_gb300 import capi, units
 from spectrum_gb300 import workloads as W
 from spectrum_gb300.datacontainer import DataContainer as DC
-from spectrum_gb300.plugins import BoundaryPlaneAbsorb, BoundaryPlaneReflect, DiffusionRigidityMagneticFieldPowerLaw
+from spectrum_gb300.plugins import (BoundaryPlaneAbsorb, BoundaryPlaneReflect, DiffusionRigidityMagneticFieldPowerLaw,
+                                    InitialMomentumLogEnergyPitchBand)
 from spectrum_gb300.simulation import open_problems, run_problems
 
 pytestmark = pytest.mark.gpu
@@ -176,3 +178,32 @@ def test_guiding_repacking_keeps_the_orbits(built_lib, n):
         assert np.array_equal(a.records[0][f], b.records[0][f]), f
     for (ca, _, na), (cb, _, nb) in zip(a.distros[0], b.distros[0]):
         assert na == nb and np.array_equal(ca, cb)
+
+
+INITIAL_MOMENTA = {
+    "beam": (cases.InitialMomentumBeam(), DC().double(1.0)),
+    "ring": (cases.InitialMomentumRing(), DC().double(1.0).double(0.7)),
+    "shell": (cases.InitialMomentumShell(), DC().double(1.0)),
+    "thick_shell": (cases.InitialMomentumThickShell(), DC().double(0.5).double(2.0).bool(False)),
+    "thick_shell_log": (cases.InitialMomentumThickShell(), DC().double(0.5).double(2.0).bool(True)),
+    "maxwell": (cases.InitialMomentumMaxwell(), DC().double(1.0).double(0.3).double(0.2)),
+    "pitch_band": (InitialMomentumLogEnergyPitchBand(), DC().double(0.5).double(2.0).double(-0.5).double(0.5)),
+}
+
+
+@pytest.mark.parametrize("precision", [capi.SPX_FP64, capi.SPX_MIXED])
+@pytest.mark.parametrize("traj,name", [
+    (t, n) for t in (cases.TRAJ_PARKER, cases.TRAJ_LORENTZ, cases.TRAJ_GUIDING, cases.TRAJ_FOCUSED, cases.TRAJ_FIELDLINE)
+    for n in sorted(INITIAL_MOMENTA) if n not in {cases.TRAJ_PARKER: ("beam", "ring"),
+                                                  cases.TRAJ_FIELDLINE: ("beam", "ring", "pitch_band")}.get(t, ())])
+def test_initial_momenta_match_oracle(built_lib, traj, name, precision):
+    """A start samples its momentum twice; where the first sample is only counted, the second takes the same draws.
+    FP32 kernels hold the field direction, which some samples follow, to 2**-24 per component; FP64 differs from the
+    oracle by the libraries' last bits."""
+    bg = (cases.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((0, 0, 0)).vec((0.3, -0.2, 0.8)).double(0.05))
+    pb = cases._parker(n=70, traj=traj, bg=bg, diff=None if traj == cases.TRAJ_PARKER else False, t_end=0.01,
+                       is_=(cases.InitialSpaceFixed(), DC().vec((0.1, 0.2, 0.3))), im=INITIAL_MOMENTA[name])
+    rec, ref = run_problems(pb, precision=precision, record=True).records[0], ot.run_oracle(pb).traj
+    scale = np.linalg.norm(ref["mom0"], axis=1, keepdims=True)
+    tol = 1e-13 if precision == capi.SPX_FP64 else 1e-6
+    assert np.all(np.abs(rec["mom0"] - ref["mom0"]) <= tol * scale)
