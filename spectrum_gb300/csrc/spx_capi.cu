@@ -470,12 +470,12 @@ void set_rk(const spx_ctx* c, spx::RunConfig& cfg)
 // Trajectories per lane of the deep build (58,368 lanes on a GB300) up to which an untuned FP32 run takes it.
 // Measured, wide against deep build: in a uniform field trajectories take the same steps and a launch has no
 // drain to speak of (3e4 trajectories 1.52 / 1.08 ms, 6e4 1.59 / 2.09, 1e6 15.3 / 18.2): one per lane. Lorentz
-// orbits in the dipole (2e5 42.3 / 39.8 ms, 4e5 60.3 / 63.2): five. Parker trajectories elsewhere differ in
+// orbits in the dipole (4e5 42.0 / 38.5 ms, 1e6 72.5 / 75.0): ten. Parker trajectories elsewhere differ in
 // length by a factor of ten and more, and the drain lasts as long as the longest (modulation, 1.9e5: 205 /
 // 143 ms, 1.28e6: 411 / 371; shock, 8e5: 151 / 148; grid, 6.4e5: 250 / 206): twenty.
 int64_t deep_lanes_limit(const spx_ctx* c)
 {
-   return c->traj == SPX_TRAJ_LORENTZ ? 5 : (c->bg_kind == spx::kBgUniform ? 1 : 20);
+   return c->traj == SPX_TRAJ_LORENTZ ? 10 : (c->bg_kind == spx::kBgUniform ? 1 : 20);
 }
 
 // The launch shape of a run: the caller's, else the one spx_autotune chose, else the defaults (the

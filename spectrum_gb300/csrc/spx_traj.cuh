@@ -2049,6 +2049,14 @@ constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
 // grid transport 366 ms at 32, 355 at 64).
 constexpr int kDrainSteps = 64;
 
+// The FP32 Lorentz kernels start trajectories several at a time. A start is FP64 work that holds its warp as long for
+// one lane as for all of them, and at a thousand steps an orbit a lane of the warp ends every thirty: starts took a
+// quarter of the time. A lane waits until kRefillLanes of its warp are idle, about kWaitSteps steps at the most, so that
+// orbits far longer than that lose nothing. Dipole, 2e5 orbits 30.2 -> 25.9 ms, 4e5 50.0 -> 42.0, 1e6 94.9 -> 72.5
+// (128 steps: 26.3, 42.9, 75.2). Guiding centres gained 5% at 5e5 and lost 5% below
+// 1e5; Parker and focused trajectories are longer, and start too rarely for it to show.
+constexpr int kRefillLanes = 16;
+
 template <int TT, int BG, class R, int DM, bool GT, int DK, int BL, int MB>
 __global__ void __launch_bounds__(128, MB)
 step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict__ Pd, RunConfig cfg,
@@ -2087,12 +2095,14 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
    constexpr bool kRepack = MB != kWideBlocksF32 || TT == kGuiding;
    // what shortens a lone warp's step at the cost of registers: not in the wide build of the Parker kernels
    constexpr bool kShortChain = MB != kWideBlocksF32;
+   constexpr int kWaitSteps = sizeof(R) == 4 && TT == kLorentz ? 256 : 0;
    __shared__ unsigned long long s_buf[kRepack ? 128 : 1];
    __shared__ volatile int s_dry;
    if constexpr (kRepack) {
       if (threadIdx.x == 0) s_dry = !queue;
       __syncthreads();
    }
+   [[maybe_unused]] int waited = 0;  // steps since the warp has had idle lanes
    [[maybe_unused]] bool drain = false;
    [[maybe_unused]] int live = blockDim.x >> 5;  // warps that may hold trajectories
    int K = cfg.steps_per_sync > 0 ? cfg.steps_per_sync : 1;
@@ -2100,7 +2110,13 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
       if (queue && !drain) {
          // refill idle lanes from the work queue: one atomic per warp
          unsigned idle = __ballot_sync(0xffffffffu, !active);
-         if (idle) {
+         bool refill = idle != 0;
+         if constexpr (kWaitSteps > 0) {
+            waited = idle ? waited + K : 0;
+            refill = __popc(idle) >= kRefillLanes || waited > kWaitSteps;
+            if (refill) waited = 0;
+         }
+         if (refill) {
             int lane = threadIdx.x & 31;
             int leader = __ffs(idle) - 1;
             unsigned long long base = 0;

@@ -207,3 +207,16 @@ def test_initial_momenta_match_oracle(built_lib, traj, name, precision):
     scale = np.linalg.norm(ref["mom0"], axis=1, keepdims=True)
     tol = 1e-13 if precision == capi.SPX_FP64 else 1e-6
     assert np.all(np.abs(rec["mom0"] - ref["mom0"]) <= tol * scale)
+
+
+@pytest.mark.parametrize("n,tuning", [(1, (64, 0, 8, 1)), (65, (64, 1, 8, 1)), (20_000, (64, 1, 8, 1)), (20_000, (64, 1, 1000, 1)),
+                                      (20_000, (32, 1, 1, 1)), (20_000, (128, 1, 8, 1))])
+def test_lanes_that_wait_for_a_start_change_no_orbit(built_lib, n, tuning):
+    """FP32 Lorentz orbits on one block of lanes that start several orbits at a time, at most a few hundred steps late,
+    against the plain grid, which has every orbit started at once: final states bit for bit."""
+    pb = W.dipole_orbits(n_traj=n, t_end=0.2 / units.unit_time)
+    a = run_problems(pb, precision=capi.SPX_MIXED, record=True, tuning=capi.Tuning(*tuning))
+    b = run_problems(pb, precision=capi.SPX_MIXED, record=True, tuning=capi.Tuning(128, 0, 8, 0))
+    assert a.stats.steps == b.stats.steps and a.stats.events == b.stats.events
+    for f in ("attempts", "status", "steps", "t", "pos", "mom", "pos0", "mom0"):
+        assert np.array_equal(a.records[0][f], b.records[0][f]), f
