@@ -16,6 +16,7 @@ import pytest
 import oracle_tools as ot
 import test_oracle_plugins as cases
 from spectrum_gb300 import capi, units
+from spectrum_gb300 import plugins as P
 from spectrum_gb300 import workloads as W
 from spectrum_gb300.datacontainer import DataContainer as DC
 from spectrum_gb300.plugins import (BoundaryPlaneAbsorb, BoundaryPlaneReflect, DiffusionRigidityMagneticFieldPowerLaw,
@@ -220,3 +221,22 @@ def test_lanes_that_wait_for_a_start_change_no_orbit(built_lib, n, tuning):
     assert a.stats.steps == b.stats.steps and a.stats.events == b.stats.events
     for f in ("attempts", "status", "steps", "t", "pos", "mom", "pos0", "mom0"):
         assert np.array_equal(a.records[0][f], b.records[0][f]), f
+
+
+@pytest.mark.parametrize("n_distros", [0, 1])
+@pytest.mark.parametrize("precision", [capi.SPX_FP64, capi.SPX_MIXED])
+def test_problems_added_after_a_run_get_buffers_of_their_own(built_lib, precision, n_distros):
+    """The problem buffers of a context are one allocation: problems added after a run, with bins of their own or with
+    no distribution at all, are in the next run as if they had been there from the first."""
+    pb = cases._parker(n=40, t_end=0.05, is_=(cases.InitialSpaceFixed(), DC().vec((0.3, 0, 0))))
+    pb.plugins = [e for e in pb.plugins if n_distros or e.plugin.role != P.ROLE_DISTRIBUTION]
+    out = []
+    for before in (1, 3):
+        sim = open_problems([pb] * before, precision=precision, record=True)
+        sim.MainLoop()
+        for k in range(before, 3):
+            sim.ctx.add_problem(pb.n_traj, pb.seed)
+        sim.ctx.run()
+        out.append((sim.ctx.sync().steps, [sim.ctx.records(k, 40)["pos"] for k in range(3)]))
+        sim.close()
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
