@@ -85,8 +85,9 @@ extern "C" {
                                        1 Milstein, 2 RK2 */
 #define SPX_OPT_SPECIALIZE 10       /* 1 (default): SPX_MIXED Parker contexts whose problems share the diffusion class
                                        FullConstant or RigidityMagneticFieldPowerLaw run on kernels compiled for that
-                                       class, and, where every problem has one expiry or pass time boundary, two
-                                       spheres and no momentum boundary, for that layout; 2: for the class only;
+                                       class, and for the boundary layout where every problem has one expiry or
+                                       pass time boundary and two spheres, or (FullConstant) two planes and one
+                                       injection or pass momentum boundary, or nothing else; 2: for the class only;
                                        0: on the kernel that dispatches at run time. 1 and 2 also run SPX_MIXED
                                        TrajectoryGuiding contexts on kernels without the scattering and
                                        perpendicular steps of the other guiding-centre types. The Parker kernels
