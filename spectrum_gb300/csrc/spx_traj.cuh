@@ -554,7 +554,9 @@ __device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL =
 
 // CL: moved() is no less than the distance moved since the last call: while the clearance lasts no spatial
 // boundary can have been crossed, and none is evaluated (a state's delta_old is then an older one of the same sign;
-// of an absorbing or passing boundary only the sign is read). One GB300: focused transport 326 -> 286 ms, shock
+// of an absorbing or passing boundary only the sign is read). In double it is the difference of the positions: the
+// increments fall short of it by their rounding, which a field that drives every step alike adds up. (The sums of the
+// float kernels lose 2^-48 of the position a step, in 10^7 steps a thousandth of bnd_clearance's margin.) One GB300: focused transport 326 -> 286 ms, shock
 // acceleration 286 -> 268 ms, modulation 245 -> 238 ms. Not in the wide FP32 Parker kernels, whose warps wait for issue
 // slots and registers, not for the evaluation (modulation with every lane busy 4.84e10 -> 4.61e10 steps/s with it).
 template <int TT, int BL, bool CL, class R, class A, class F>
@@ -912,10 +914,10 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    V3<R> dr = from_basis(mk(h.sperp * dWx, h.sperp * dWy, h.spara * dWz), h.fa);
    R dts = L.dt * R(1);
    acc_add(L.t, fwd ? L.dt : -L.dt);
-   V3<R> d;
+   [[maybe_unused]] const V3<R> pos = val3<R>(L.pos);
+   [[maybe_unused]] V3<R> d;
    if constexpr (kFP64) {
-      d = (fwd ? dts : -dts) * h.slope;
-      add3(L.pos, d);
+      add3(L.pos, (fwd ? dts : -dts) * h.slope);
       add3(L.pos, dr);
    }
    else {
@@ -930,7 +932,7 @@ __device__ __forceinline__ void parker_uniform_advance(Lane<R, A>& L, BndView<R>
    sp.region = mk(R(1), R(1), R(1));
    sp.Bmag = h.Bmag;
    sp.divU = h.divU;
-   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
+   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return norm1(kFP64 ? val3<R>(L.pos) - pos : d); });
    L.steps++;
 }
 
@@ -1020,12 +1022,11 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    V3<R> dr = from_basis(mk(sperp * dWx, sperp * dWy, spara * dWz), fa);
    // RKStep with the Euler table, then the stochastic displacement
    R dts = L.dt * R(1);
-   V3<R> d;
+   [[maybe_unused]] V3<R> d;
    if (fwd) {
       acc_add(L.t, L.dt);
       if constexpr (kFP64) {
-         d = dts * slope;
-         add3(L.pos, d);
+         add3(L.pos, dts * slope);
          acc_add(L.mom.x, dts * slope_p);
          add3(L.pos, dr);
       }
@@ -1038,8 +1039,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
    else {
       acc_add(L.t, -L.dt);
       if constexpr (kFP64) {
-         d = (-dts) * slope;
-         add3(L.pos, d);
+         add3(L.pos, (-dts) * slope);
          acc_add(L.mom.x, -(dts * slope_p));
          add3(L.pos, dr);
       }
@@ -1050,7 +1050,7 @@ __device__ __forceinline__ void parker_advance(Lane<R, A>& L, BndView<R> bv, Sta
       }
    }
    if (sa != R(0)) L.amp += dts * sa * m_exp(L.wgt);
-   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return kFP64 ? norm1(d) + norm1(dr) : norm1(d); });
+   handle_boundaries<kParker, BL, CL>(L, bv, sp, s0, P, Pd, S, [&] { return norm1(kFP64 ? val3<R>(L.pos) - pos : d); });
    L.steps++;
 }
 

@@ -2,7 +2,8 @@
 
 - Quotients by a shared divisor leave their fast form where an exponent could over- or underflow: a dmax of
   1e140 takes the time-step bounds there (FP64 against the oracle).
-- Stage points told by their clearance from the boundaries, against the oracle's evaluation of each.
+- Stage points told by their clearance from the boundaries, against the oracle's evaluation of each; steps so small
+  that the positions' rounding is a part of the way, against the step count that arithmetic gives.
 - The FP32 kernels compiled for a boundary layout against the one that reads it from the descriptor.
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - The initial momentum, of whose two samples the first is only counted where nothing reads it, against the oracle.
@@ -240,3 +241,24 @@ def test_problems_added_after_a_run_get_buffers_of_their_own(built_lib, precisio
         out.append((sim.ctx.sync().steps, [sim.ctx.records(k, 40)["pos"] for k in range(3)]))
         sim.close()
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("ulps", [20.51, 20.49, 3.6])
+@pytest.mark.parametrize("flow", [cases.FORWARD, cases.BACKWARD])
+@pytest.mark.parametrize("diffusion", ["held", "general"])
+def test_rounding_of_small_steps_moves_no_crossing(built_lib, diffusion, flow, ulps):
+    """FP64 Parker steps of some units in the last place of the position, all rounded the same way: a path without
+    diffusion moves ``round(ulps)`` units a step, and ends at the step that reaches the absorbing plane."""
+    c, ulp = cases, 2.0 ** -52
+    u = 1.0 if flow == c.FORWARD else -1.0
+    bg = (c.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((u, 0, 0)).vec((1.0, 0, 0)).double(2.0 * ulps * ulp))
+    diff = (c.DiffusionFullConstant(), DC().double(0.0).double(0.0)) if diffusion == "held" else \
+           (c.DiffusionKineticEnergyRadialDistancePowerLaw(),
+            DC().double(0.0).double(1.0).double(0.2).double(0.5).double(1.0).double(0.1).int(0).double(1.0).double(0.1).double(4.0))
+    units_away = 200_000
+    pb = c._parker(n=3, bg=bg, diff=diff, flow=flow, t_end=0.2 if flow == c.FORWARD else -0.2,
+                   is_=(c.InitialSpaceFixed(), DC().vec((1.0, 0, 0))),
+                   bnds=[(BoundaryPlaneAbsorb(), c.B(DC(), 1, [0]).vec((1.0 + units_away * ulp, 0, 0)).vec((1.0, 0, 0)))])
+    rec = run_problems(pb, precision=capi.SPX_FP64, record=True).records[0]
+    assert np.array_equal(rec["steps"], ot.run_oracle(pb).traj["steps"])
+    assert np.all(np.abs(rec["steps"].astype(np.int64) - -(-units_away // round(ulps))) <= 1)
