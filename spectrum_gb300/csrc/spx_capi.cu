@@ -106,6 +106,7 @@ struct spx_ctx {
    double* d_rwts = nullptr;
    unsigned long long* d_rn = nullptr;
    int64_t n_rvals = 0, n_rwts = 0;
+   int n_rn = 0;  // problems that d_rn holds
 };
 
 namespace {
@@ -144,6 +145,7 @@ void free_buffers(spx_ctx* c)
    c->d_rwts = nullptr;
    c->d_rn = nullptr;
    c->n_rvals = c->n_rwts = 0;
+   c->n_rn = 0;
    c->d_ctr = nullptr;
    c->d_rec = nullptr;
    c->rec_cap = 0;
@@ -237,6 +239,7 @@ int upload(spx_ctx* c)
       c->d_rvals = c->d_rwts = nullptr;
       c->d_rn = nullptr;
       c->n_rvals = c->n_rwts = 0;
+      c->n_rn = 0;
       if (rv > 0) {
          SPX_CUDA(cudaMalloc(&c->d_rvals, sizeof(double) * rv));
          SPX_CUDA(cudaMalloc(&c->d_rwts, sizeof(double) * rw));
@@ -244,6 +247,7 @@ int upload(spx_ctx* c)
          SPX_CUDA(cudaMemsetAsync(c->d_rn, 0, sizeof(unsigned long long) * n * spx::kMaxDistro, c->stream));
          c->n_rvals = rv;
          c->n_rwts = rw;
+         c->n_rn = n;
       }
    }
    std::vector<spx::ProblemDesc> hd(n);
@@ -1262,9 +1266,9 @@ int spx_reset_distributions(spx_ctx_t c)
    if (c->d_counts == nullptr) return SPX_OK;
    SPX_CUDA(cudaMemsetAsync(c->d_counts, 0, sizeof(int32_t) * std::max<int64_t>(c->n_counts, 1), c->stream));
    SPX_CUDA(cudaMemsetAsync(c->d_sums, 0, sizeof(double) * std::max<int64_t>(c->n_sums, 1), c->stream));
-   SPX_CUDA(cudaMemsetAsync(c->d_nev, 0, sizeof(unsigned long long) * c->problems.size() * spx::kMaxDistro, c->stream));
-   if (c->d_rn)
-      SPX_CUDA(cudaMemsetAsync(c->d_rn, 0, sizeof(unsigned long long) * c->problems.size() * spx::kMaxDistro, c->stream));
+   // as many problems as the buffers hold: those added since the last run have none yet
+   SPX_CUDA(cudaMemsetAsync(c->d_nev, 0, sizeof(unsigned long long) * c->n_desc * spx::kMaxDistro, c->stream));
+   if (c->d_rn) SPX_CUDA(cudaMemsetAsync(c->d_rn, 0, sizeof(unsigned long long) * c->n_rn * spx::kMaxDistro, c->stream));
    SPX_CUDA(cudaStreamSynchronize(c->stream));
    return SPX_OK;
 }
