@@ -226,13 +226,16 @@ int upload(spx_ctx* c)
    if (grid_missing(c)) return SPX_ERR_STATE;
    // record buffers of the keep_records distributions (DistributionBase::AddRecord)
    int64_t rv = 0, rw = 0;
+   int keeping = 0;  // problems up to the last one that keeps records
    for (int k = 0; k < n; k++)
       for (int d = 0; d < c->problems[k].pd.nd; d++)
          if (c->problems[k].pd.d[d].keep_records) {
             rv += 3 * c->rec_capacity;
             rw += (int64_t)c->problems[k].pd.d[d].width * c->rec_capacity;
+            keeping = k + 1;
          }
-   if (rv != c->n_rvals || rw != c->n_rwts || (rv > 0 && c->d_rn == nullptr)) {
+   // (twice the problems at half the capacity take as many slots, but more counters)
+   if (rv != c->n_rvals || rw != c->n_rwts || (rv > 0 && (c->d_rn == nullptr || keeping > c->n_rn))) {
       cudaFree(c->d_rvals);
       cudaFree(c->d_rwts);
       cudaFree(c->d_rn);

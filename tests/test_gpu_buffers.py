@@ -36,3 +36,24 @@ def test_reset_between_added_problems_and_the_next_run(built_lib, added):
     finally:
         a.close()
         b.close()
+
+
+def test_more_problems_at_a_smaller_record_capacity(built_lib):
+    """Forty problems that keep a tenth of the records of four take as many slots, and ten times the counters."""
+    pb = CASES["focused_fwd_slab_records"]
+    a, b = open_problems([pb] * 4, capi.SPX_FP64), open_problems([pb] * 40, capi.SPX_FP64)
+    try:
+        a.ctx.set_option(capi.SPX_OPT_RECORD_CAPACITY, 100)
+        a.MainLoop()
+        for _ in range(36):
+            a.ctx.add_problem(pb.n_traj, pb.seed)
+        b.ctx.set_option(capi.SPX_OPT_RUN_INDEX, 1)
+        for sim in (a, b):
+            sim.ctx.set_option(capi.SPX_OPT_RECORD_CAPACITY, 10)
+            sim.ctx.run()
+            sim.ctx.sync()
+        for (da, ra), (db, rb) in zip(_state(a, 40), _state(b, 40)):
+            assert ra == rb == da[2] == db[2] and np.array_equal(da[0], db[0])
+    finally:
+        a.close()
+        b.close()
