@@ -109,11 +109,15 @@ extern "C" {
 /* ---- types ----------------------------------------------------------------------------- */
 typedef struct spx_ctx* spx_ctx_t;
 
+/* A launch shape: how fast a run is, never what it computes. Two shapes stand for launches of few trajectories
+ * wherever such a launch is theirs: {128, *, *, 1} in SPX_MIXED runs the kernels' deep build, and {32, *, *, 0} in SPX_FP64
+ * spreads the trajectories over the schedulers, several lanes each where that helps. */
 typedef struct {
-   int block_size;      /* threads per block; 0 = autotuned */
-   int blocks_per_sm;   /* resident blocks per SM for the persistent launch; 0 = autotuned */
-   int steps_per_sync;  /* steps between lane refills of the work queue; 0 = autotuned */
-   int schedule;        /* 0 = one thread per trajectory (plain grid), 1 = persistent work queue */
+   int block_size;      /* threads per block, 32 to 128; 0 = 128 */
+   int blocks_per_sm;   /* resident blocks per SM for the persistent launch; 0 = as many as fit */
+   int steps_per_sync;  /* steps between lane refills of the work queue; 0 = 16. Kernels that repack the lanes of a block
+                           do so every 64 steps once the queue is empty, and from the start in the plain grid */
+   int schedule;        /* 0 = plain grid, every trajectory started at once, 1 = persistent work queue */
 } spx_tuning;
 
 typedef struct {
@@ -194,7 +198,8 @@ int spx_set_background_blocks(spx_ctx_t ctx, const int32_t n_blocks[3], const do
 void spx_grid_units(double out[4]);
 
 /* Integrate every trajectory of every problem; replaces MainLoop (src/simulation.cc:818-835).
- * Enqueues on the context stream and returns; tuning may be NULL (autotuned). Each call draws
+ * Enqueues on the context stream and returns; tuning may be NULL (the shape of few trajectories where
+ * the run has few, else the spx_autotune result, else a default). Each call draws
  * fresh trajectory ids, so repeated calls add new trajectories to the distributions. */
 int spx_run(spx_ctx_t ctx, const spx_tuning* tuning);
 
@@ -204,8 +209,10 @@ int spx_sync(spx_ctx_t ctx, spx_stats* stats);
 /* Choose the launch shape (block size, refill interval, schedule) by timing candidates on a sample
  * of the context's problems: about sample_traj trajectories (0: two per resident lane), each
  * stopped after 2048 steps, on separate buffers and random streams. spx_run with a NULL tuning
- * then uses the fastest; best (may be NULL) receives it. No reference counterpart: the
- * reference's MPI farm has no launch shape to tune. */
+ * then uses the fastest, except for launches of few trajectories (SPX_MIXED: up to 20 a lane of the kernels' deep
+ * build, 10 for Lorentz orbits, 1 in a uniform field; SPX_FP64: up to a warp per scheduler), whose shape the
+ * samples cannot judge and which keep it. best (may be NULL) receives the shape that spx_run with a NULL tuning uses
+ * for the present problems. No reference counterpart: the reference's MPI farm has no launch shape to tune. */
 int spx_autotune(spx_ctx_t ctx, int64_t sample_traj, spx_tuning* best);
 
 /* Size of the fixed device array spx_run_static works in (every GPU that loads the library holds
@@ -224,8 +231,7 @@ int spx_autotune(spx_ctx_t ctx, int64_t sample_traj, spx_tuning* best);
  * problem descriptors live in a fixed array of SPX_STATIC_SCRATCH_BYTES; a context whose
  * descriptors do not fit is rejected with SPX_ERR_TOO_LARGE. The call allocates no device memory
  * (no cudaMalloc, cudaFree or allocating library routine); it blocks until the launch is done
- * and fills stats (may be NULL). The launch shape is chosen as spx_run chooses it (tuning, else the
- * spx_autotune result, else the defaults). The first call on a device looks up the array's address
+ * and fills stats (may be NULL). The launch shape is chosen as spx_run chooses it. The first call on a device looks up the array's address
  * there (and may load the library's device code), so make it before any stream capture; the
  * address is kept for the life of the process, so resetting the device (cudaDeviceReset) while the
  * library is loaded is not supported. All calls share

@@ -176,7 +176,7 @@ class Context:
 
     def autotune(self, sample_traj: int = 0) -> Tuning:
         """spx_autotune: time candidate launch shapes on a sample; later runs without a tuning use
-        the fastest."""
+        the fastest, launches of few trajectories the shape that is theirs. Returns what such a run takes now."""
         t = Tuning()
         check(self.lib.spx_autotune(self._h, int(sample_traj), ctypes.byref(t)), "spx_autotune")
         return t

@@ -487,71 +487,74 @@ int64_t deep_lanes_limit(const spx_ctx* c)
    return c->traj == SPX_TRAJ_LORENTZ ? 10 : (c->bg_kind == spx::kBgUniform ? 1 : 20);
 }
 
-// The launch shape of a run: the caller's, else the one spx_autotune chose, else the defaults (the
-// FP64 drop-in keeps one thread per trajectory; the FP32 stepper takes the persistent queue in
-// blocks of 64 refilled every 8 steps, the shape that measured fastest on the modulation batch, or up to
-// deep_lanes_limit the kernels' deep build in blocks of 128, whose warps it repacks; the guiding centres' kernels
-// repack in their one build).
-// Unset fields are completed and checked; blocks per SM is capped by the kernel's occupancy for
-// "slots" boundary states per lane. Shared by spx_run and spx_run_static.
-int resolve_tuning(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t total, spx_tuning& tu, bool& deep)
+// Blocks per SM of the deep build where an FP32 run of "total" trajectories takes it, else 0.
+int deep_blocks(spx_ctx* c, int slots, int64_t total)
 {
-   tu = spx_tuning{};
-   deep = false;
+   if (c->precision != SPX_MIXED) return 0;
+   const int occ = occupancy(c, 128, slots, true);
+   return total <= deep_lanes_limit(c) * c->sm_count * 128 * occ ? occ : 0;
+}
+
+// How a run is launched: the shape that its statistics report, and what follows from it.
+struct LaunchShape {
+   spx_tuning tu;
+   bool deep;              // the FP32 kernels' deep build
+   int64_t grid;
+   int warp_lanes, team;   // the plain grid: lanes of a warp that hold trajectories, in FP64 in teams of "team" lanes
+};
+
+// The launch shape of a run: the caller's, else that of few trajectories, else the one spx_autotune chose, else the
+// defaults (the FP64 drop-in keeps one thread per trajectory; the FP32 stepper takes the persistent queue in
+// blocks of 64 refilled every 8 steps, the shape that measured fastest on the modulation batch; the guiding centres'
+// kernels repack their blocks, of 128). Unset fields are completed and checked; blocks per SM is capped by the kernel's
+// occupancy for "slots" boundary states per lane. Shared by spx_run and spx_run_static.
+//
+// Few trajectories. FP32, up to deep_lanes_limit: the deep build, in queue blocks of 128, whose warps it repacks.
+// FP64, up to one warp per scheduler: the plain grid in blocks of 32. The FP64 pipe takes a warp instruction
+// every 64 cycles of each scheduler, whatever its active lanes, so one warp per scheduler is free: such a launch
+// spreads over all schedulers (fewer trajectories a warp diverge less), and where the kernel evaluates finite
+// differences or pairs of normals its trajectories get up to eight lanes each, in the dipole four (a component each).
+// The autotuner's samples, two trajectories a lane cut before they end, have no drain and full warps: what it
+// finds holds for the launches above. A shape given by the caller that is the one of few trajectories
+// is run as such, so what a run reports, or spx_autotune returns, runs the same when it is given back; any other
+// has the wide build and full warps of one lane a trajectory.
+int resolve_shape(spx_ctx* c, const spx_tuning* tuning, int slots, int64_t total, LaunchShape& s)
+{
+   const bool mixed = c->precision == SPX_MIXED;
+   const int64_t warps = (int64_t)c->sm_count * 4;  // one per scheduler
+   const bool few = !mixed && total <= warps * 32;
+   spx_tuning& tu = s.tu;
+   int occ = 0;
    if (tuning) tu = *tuning;
+   else if ((occ = deep_blocks(c, slots, total)) > 0) tu = spx_tuning{128, 0, 8, 1};
+   else if (few) tu = spx_tuning{32, 0, 0, 0};
    else if (c->has_tuned) tu = c->tuned;
-   else {
-      tu.schedule = c->precision == SPX_MIXED ? 1 : 0;
-      if (tu.schedule) {
-         const bool guiding = c->traj >= SPX_TRAJ_GUIDING && c->traj <= SPX_TRAJ_GUIDING_DIFF_SCATT;
-         tu.block_size = guiding ? 128 : 64;  // the guiding centres' kernels repack their blocks
-         tu.steps_per_sync = 8;
-         const int occ = occupancy(c, 128, slots, true);
-         if (occ > 0 && total <= deep_lanes_limit(c) * c->sm_count * 128 * occ) {
-            deep = true;
-            tu.block_size = 128;
-         }
-      }
-   }
+   else if (!mixed) tu = spx_tuning{};
+   else tu = spx_tuning{c->traj >= SPX_TRAJ_GUIDING && c->traj <= SPX_TRAJ_GUIDING_DIFF_SCATT ? 128 : 64, 0, 8, 1};
    if (tu.schedule != 0 && tu.schedule != 1) return SPX_ERR_INVALID_ARG;
    if (tu.block_size <= 0) tu.block_size = 128;
    if (tu.block_size % 32 || tu.block_size > 128) return SPX_ERR_INVALID_ARG;
    if (tu.steps_per_sync <= 0) tu.steps_per_sync = tu.schedule ? 16 : 1 << 30;
-   int occ = occupancy(c, tu.block_size, slots, deep);
-   if (occ <= 0) occ = 1;
+   if (tuning && tu.schedule == 1 && tu.block_size == 128) occ = deep_blocks(c, slots, total);
+   s.deep = occ > 0;
+   if (!s.deep) occ = std::max(occupancy(c, tu.block_size, slots, false), 1);
    if (tu.blocks_per_sm <= 0 || tu.blocks_per_sm > occ) tu.blocks_per_sm = occ;
-   return SPX_OK;
-}
-
-// The plain grid of a run: how many lanes of a warp hold trajectories, and in FP64 how many lanes share one.
-// The FP64 pipe takes a warp instruction every 64 cycles of each scheduler, whatever its active lanes, so up to
-// one warp per scheduler is free: a launch that fits spreads over all schedulers (fewer trajectories a warp
-// diverge less), and where the kernel evaluates finite differences or pairs of normals its trajectories
-// get up to eight lanes each, in the dipole four (a component each). Larger launches take one lane each and full warps; a caller's own launch shape
-// is kept as given.
-struct PlainShape {
-   int64_t grid;
-   int block, warp_lanes, team;
-};
-
-PlainShape plain_shape(const spx_ctx* c, int64_t total, int block, bool chosen_here)
-{
-   PlainShape s{0, block, 32, 1};
-   const int64_t warps = (int64_t)c->sm_count * 4;  // one per scheduler
-   if (chosen_here && c->precision == SPX_FP64 && total <= warps * 32) {
+   s.warp_lanes = 32;
+   s.team = 1;
+   if (few && tu.schedule == 0 && tu.block_size == 32) {
       const bool parker = c->traj == SPX_TRAJ_PARKER || c->traj == SPX_TRAJ_PARKER_SOURCE;
       const bool fd = c->deriv_mode == 0 && c->bg_kind == spx::kBgSolarWind;
       const bool split = c->bg_kind == spx::kBgDipole && (c->traj == SPX_TRAJ_LORENTZ || c->traj == SPX_TRAJ_GUIDING);
       const int most = parker || fd ? 8 : (split ? 4 : 1);
       while (s.team < most && total * s.team * 2 <= warps * 32) s.team *= 2;
       s.warp_lanes = s.team * (int)std::max<int64_t>(1, (total + warps - 1) / warps);
-      s.block = 32;
    }
-   const int64_t per_block = (int64_t)(s.block / 32) * (s.warp_lanes / s.team);
-   s.grid = (total + per_block - 1) / per_block;
-   return s;
+   const int64_t per_block = (int64_t)(tu.block_size / 32) * (s.warp_lanes / s.team);
+   s.grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm  // persistent: fill the GPU once
+                             : (total + per_block - 1) / per_block;
+   s.grid = std::max<int64_t>(1, std::min<int64_t>(s.grid, 0x7fffffff));
+   return SPX_OK;
 }
-
 
 // What a captured graph depends on: launch shape, the run configuration apart from the run
 // index, and the device buffers. A different key means a new capture.
@@ -1008,19 +1011,17 @@ int spx_run(spx_ctx_t c, const spx_tuning* tuning)
       int rc = upload(c);
       if (rc != SPX_OK) return rc;
    }
-   spx_tuning tu;
    const int slots = bnd_slots(c);
-   spx::LaunchArgs a;
-   const int trc = resolve_tuning(c, tuning, slots, c->total_traj, tu, a.deep);
+   LaunchShape shape;
+   const int trc = resolve_shape(c, tuning, slots, c->total_traj, shape);
    if (trc != SPX_OK) return trc;
-   const PlainShape ps = plain_shape(c, c->total_traj, tu.block_size, tuning == nullptr && !c->has_tuned);
-   if (tu.schedule == 0) tu.block_size = ps.block;
+   const spx_tuning& tu = shape.tu;
+   spx::LaunchArgs a;
    a.block = dim3(tu.block_size);
-   int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm : ps.grid;  // persistent: fill the GPU once
-   grid = std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff));
-   a.cfg.warp_lanes = ps.warp_lanes;
-   a.cfg.team = ps.team;
-   a.grid = dim3((unsigned)grid);
+   a.deep = shape.deep;
+   a.cfg.warp_lanes = shape.warp_lanes;
+   a.cfg.team = shape.team;
+   a.grid = dim3((unsigned)shape.grid);
    a.stream = c->stream;
    a.problems_r = c->d_pr;
    a.problems_d = c->d_pd;
@@ -1066,7 +1067,8 @@ int spx_run(spx_ctx_t c, const spx_tuning* tuning)
 // The autotuner: time candidate launch shapes on a sample of the context's problems (each problem
 // keeps its share of trajectories, every trajectory stops after a fixed number of steps) and keep
 // the fastest by accepted steps per second. The sample runs on buffers of its own with other
-// random streams, so the context's distributions and trajectory ids are untouched.
+// random streams, so the context's distributions and trajectory ids are untouched. The samples have full warps of the
+// wide build: launches of few trajectories keep the shape that resolve_shape gives them.
 int spx_autotune(spx_ctx_t c, int64_t sample_traj, spx_tuning* best)
 {
    if (!valid_ctx(c)) return SPX_ERR_INVALID_ARG;
@@ -1191,7 +1193,15 @@ int spx_autotune(spx_ctx_t c, int64_t sample_traj, spx_tuning* best)
    c->tuned = best_tu;
    c->has_tuned = true;
    c->launched = false;  // the timing events now describe a sample, not an spx_run
-   if (best) *best = best_tu;
+   if (best) {
+      // what spx_run with a NULL tuning takes now: the shape of few trajectories comes before the tuned one
+      LaunchShape shape;
+      const int rc = resolve_shape(c, nullptr, slots, total, shape);
+      if (rc != SPX_OK) return rc;
+      *best = shape.tu;
+      // (as many blocks as fit: the caller may give the shape to a larger context, whose build holds more)
+      if (shape.deep) best->blocks_per_sm = 0;
+   }
    return SPX_OK;
 }
 
@@ -1667,16 +1677,13 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    int rc = static_scratch(c->device, &scratch);
    if (rc != SPX_OK) return rc;
 
-   // launch shape: chosen as spx_run chooses it (the caller's, the autotuned one, or the defaults)
-   spx_tuning tu;
+   // launch shape: chosen as spx_run chooses it
    const int slots = bnd_slots(c);
-   spx::LaunchArgs a;
-   rc = resolve_tuning(c, tuning, slots, total, tu, a.deep);
+   LaunchShape shape;
+   rc = resolve_shape(c, tuning, slots, total, shape);
    if (rc != SPX_OK) return rc;
-   const PlainShape ps = plain_shape(c, total, tu.block_size, tuning == nullptr && !c->has_tuned);
-   if (tu.schedule == 0) tu.block_size = ps.block;
-   int64_t grid = tu.schedule == 1 ? (int64_t)c->sm_count * tu.blocks_per_sm : ps.grid;
-   grid = std::max<int64_t>(1, std::min<int64_t>(grid, 0x7fffffff));
+   const spx_tuning& tu = shape.tu;
+   spx::LaunchArgs a;
 
    // descriptors into the scratch, counters cleared
    std::vector<spx::ProblemDescT<float>> hf;
@@ -1692,9 +1699,10 @@ int spx_run_static(spx_ctx_t c, const spx_tuning* tuning, int32_t* counts, int64
    }
 
    a.block = dim3(tu.block_size);
-   a.grid = dim3((unsigned)grid);
-   a.cfg.warp_lanes = ps.warp_lanes;
-   a.cfg.team = ps.team;
+   a.deep = shape.deep;
+   a.grid = dim3((unsigned)shape.grid);
+   a.cfg.warp_lanes = shape.warp_lanes;
+   a.cfg.team = shape.team;
    a.stream = c->stream;
    a.problems_r = scratch + off_pr;
    a.problems_d = reinterpret_cast<const spx::ProblemDesc*>(scratch + off_pd);

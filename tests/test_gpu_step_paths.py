@@ -8,6 +8,8 @@
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - The initial momentum, of whose two samples the first is only counted where nothing reads it, against the oracle.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
+- Launches of few trajectories keep their shape when the autotuner has run or when a run is given back what another
+  reported; larger ones take the tuned shape.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
   and evaluated at every step (those that do), in both time flows: FP64 against the oracle, and the FP32
   kernels of one diffusion class against the kernel that dispatches at run time, whose steps are general."""
@@ -262,3 +264,45 @@ def test_rounding_of_small_steps_moves_no_crossing(built_lib, diffusion, flow, u
     rec = run_problems(pb, precision=capi.SPX_FP64, record=True).records[0]
     assert np.array_equal(rec["steps"], ot.run_oracle(pb).traj["steps"])
     assert np.all(np.abs(rec["steps"].astype(np.int64) - -(-units_away // round(ulps))) <= 1)
+
+
+def _shape(t):
+    return t.block_size, t.blocks_per_sm, t.steps_per_sync, t.schedule
+
+
+@pytest.mark.parametrize("kind,precision", [("uniform", capi.SPX_FP64), ("uniform", capi.SPX_MIXED), ("dipole", capi.SPX_FP64),
+                                            ("dipole", capi.SPX_MIXED), ("spiral", capi.SPX_MIXED)])
+def test_autotuning_leaves_few_trajectories_their_shape(built_lib, kind, precision):
+    n = 700
+    if kind == "uniform":
+        pb = W.diffusion_uniform(n_traj=n, t_end=0.02)
+    elif kind == "dipole":
+        pb = W.dipole_orbits(n_traj=n, t_end=0.01 / units.unit_time)
+    else:
+        pb = W.gcr_modulation(n_traj=n, energies_mev=[300.0], t_max_years=0.002)[0]
+    want = run_problems(pb, precision=precision, record=True)
+    sim = open_problems(pb, precision=precision, record=True)
+    try:
+        best = sim.ctx.autotune(4000)
+        shapes = []
+        for k, tuning in enumerate((None, best, want.stats.tuning)):
+            st = sim.MainLoop(tuning)
+            shapes.append(_shape(st.tuning))
+            if k == 0:
+                got = sim.ctx.records(0, n)
+    finally:
+        sim.close()
+    assert shapes == [_shape(want.stats.tuning)] * 3
+    for f in ("attempts", "status", "steps", "t", "pos", "mom"):
+        assert np.array_equal(got[f], want.records[0][f]), f
+
+
+@pytest.mark.parametrize("precision,n", [(capi.SPX_FP64, 152 * 128 + 1), (capi.SPX_MIXED, 152 * 128 * 3 + 1)])
+def test_larger_launches_take_the_tuned_shape(built_lib, precision, n):
+    """One trajectory more than the launches of few trajectories have on a GB300 (152 SMs)."""
+    sim = open_problems(W.diffusion_uniform(n_traj=n, t_end=0.005), precision=precision)
+    try:
+        best = sim.ctx.autotune(4000)
+        assert _shape(sim.MainLoop().tuning) == _shape(best) and best.blocks_per_sm > 0
+    finally:
+        sim.close()
