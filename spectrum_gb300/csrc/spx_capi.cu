@@ -487,12 +487,15 @@ int64_t deep_lanes_limit(const spx_ctx* c)
    return c->traj == SPX_TRAJ_LORENTZ ? 10 : (c->bg_kind == spx::kBgUniform ? 1 : 20);
 }
 
-// Blocks per SM of the deep build where an FP32 run of "total" trajectories takes it, else 0.
+// Blocks per SM of the deep build where an FP32 run of "total" trajectories takes it, else 0. Its occupancy, at most
+// kDeepBlocksF32 (the builds have 150 to 168 registers), is asked for where that many blocks would do: asking loads the
+// kernel (0.1 ms of a process's first run, 1.56 -> 1.44).
 int deep_blocks(spx_ctx* c, int slots, int64_t total)
 {
-   if (c->precision != SPX_MIXED) return 0;
-   const int occ = occupancy(c, 128, slots, true);
-   return total <= deep_lanes_limit(c) * c->sm_count * 128 * occ ? occ : 0;
+   const int64_t per_block = deep_lanes_limit(c) * c->sm_count * 128;
+   if (c->precision != SPX_MIXED || total > per_block * spx::kDeepBlocksF32) return 0;
+   const int occ = std::min(occupancy(c, 128, slots, true), spx::kDeepBlocksF32);
+   return total <= per_block * occ ? occ : 0;
 }
 
 // How a run is launched: the shape that its statistics report, and what follows from it.

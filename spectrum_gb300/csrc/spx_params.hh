@@ -54,6 +54,14 @@ enum BndKind : int {
 // diffusion of 1e6: 15.3 to 11.3 ms.)
 enum BndLayout : int { kLayoutAny = 0, kLayoutSpheres = 1, kLayoutPlanes = 2, kLayoutTime = 3 };
 
+// Resident blocks of 128 threads per SM the register allocation is sized for. The FP32 kernels come in two
+// builds. Wide, five blocks (20 warps, at most 102 registers), has the most steps per second with every lane
+// busy: the extra warps hide more dependent-instruction latency than the spilled values cost (four blocks ran
+// 2-5% slower). Deep, three blocks, spills nothing, so a warp's step is shorter: it is the faster one where a
+// launch is mostly its drain, the last trajectories alone on the SMs. One GB300, wide to deep with its repacking: shock acceleration of 4e4
+// trajectories 580 -> 453 ms, modulation of 1.9e5 325 -> 245 ms, on a 256^3 grid 530 -> 375 ms.
+constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
+
 enum IniKind : int {
    kItFixed = 1, kItInterval,
    kIsFixed = 10, kIsLine, kIsCircle, kIsBox, kIsSphere, kIsSphereSector, kIsRankine, kIsCylinder, kIsCylinderSector,

@@ -2024,14 +2024,6 @@ __device__ __noinline__ bool repack_lanes(LaneWords& W, Start& s0, BndView<R> bv
    return mine;
 }
 
-// Resident blocks of 128 threads per SM the register allocation is sized for. The FP32 kernels come in two
-// builds. Wide, five blocks (20 warps, at most 102 registers), has the most steps per second with every lane
-// busy: the extra warps hide more dependent-instruction latency than the spilled values cost (four blocks ran
-// 2-5% slower). Deep, three blocks, spills nothing, so a warp's step is shorter: it is the faster one where a
-// launch is mostly its drain, the last trajectories alone on the SMs. One GB300, wide to deep with its repacking: shock acceleration of 4e4
-// trajectories 580 -> 453 ms, modulation of 1.9e5 325 -> 245 ms, on a 256^3 grid 530 -> 375 ms.
-constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
-
 // One lane per thread. Dynamic shared memory holds the lanes' boundary states
 // (boundaries per lane x blockDim.x x sizeof(BndState<R>)).
 // DM is the field-derivative method (SPX_OPT_DERIV_MODE) fixed per instantiation, so the analytic
