@@ -1953,10 +1953,10 @@ __device__ __forceinline__ void start_lane(Lane<R, A>& L, BndView<R> bv, Start& 
 // lane as for 32). A block repacks at most blockDim / 32 - 1 times. Without it the deep build
 // took 499, 270 and 405 ms on the three runs given below, with it 453, 245 and 375.
 
-// Lane state as words, for the exchange below.
+// Lane state as words, for the exchange below: room for N of them.
+template <int N>
 struct LaneWords {
-   static constexpr int kMax = 48;
-   unsigned long long w[kMax];
+   unsigned long long w[N];
    int n;
    template <class T> __device__ __forceinline__ void put(const T& v)
    {
@@ -1969,7 +1969,7 @@ struct LaneWords {
 };
 
 template <class R, class A, class F>
-__device__ __forceinline__ void each_member(Lane<R, A>& L, F f)
+__device__ __forceinline__ constexpr void each_member(Lane<R, A>& L, F f)
 {
    f(L.prob); f(L.traj_id); f(L.attempt); f(L.steps); f(L.status); f(L.nrm); f(L.n_adapt);
    f(L.t);
@@ -1978,7 +1978,7 @@ __device__ __forceinline__ void each_member(Lane<R, A>& L, F f)
    f(L.amp); f(L.wgt); f(L.dt); f(L.dt_adapt); f(L.src_del_old); f(L.clear);
 }
 template <class R, class F>
-__device__ __forceinline__ void each_member(UniformStep<R>& h, F f)
+__device__ __forceinline__ constexpr void each_member(UniformStep<R>& h, F f)
 {
    int valid = h.valid;
    f(valid);
@@ -1988,11 +1988,19 @@ __device__ __forceinline__ void each_member(UniformStep<R>& h, F f)
    f(h.slope_p); f(h.sperp); f(h.spara); f(h.dtp); f(h.dmax); f(h.Bmag); f(h.divU);
    f(h.lim.none_); f(h.lim.least_); f(h.lim.error_);
 }
+template <class T>
+__device__ constexpr int count_members()
+{
+   T v{};
+   int n = 0;
+   each_member(v, [&n](const auto&) { n++; });
+   return n;
+}
 
 // Moves the words and boundary states of the block's active lanes to its first threads, in order; every
 // thread of the block takes part. Returns whether this thread holds a trajectory afterwards.
-template <class R>
-__device__ __noinline__ bool repack_lanes(LaneWords& W, Start& s0, BndView<R> bv, int slots, bool active, unsigned long long* buf)
+template <class R, int N>
+__device__ __noinline__ bool repack_lanes(LaneWords<N>& W, Start& s0, BndView<R> bv, int slots, bool active, unsigned long long* buf)
 {
    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
    const unsigned mask = __ballot_sync(0xffffffffu, active);
@@ -2012,7 +2020,8 @@ __device__ __noinline__ bool repack_lanes(LaneWords& W, Start& s0, BndView<R> bv
       if (mine) v = buf[tid];
       __syncthreads();
    };
-   for (int k = 0; k < W.n; k++) move(W.w[k]);
+#pragma unroll 1
+   for (int k = 0; k < N; k++) move(W.w[k]);
    static_assert(sizeof(Start) % 8 == 0, "Start is moved in 8-byte words");
    for (int k = 0; k < (int)(sizeof(Start) / 8); k++) move(reinterpret_cast<unsigned long long*>(&s0)[k]);
    for (int j = 0; j < slots; j++) {
@@ -2132,18 +2141,19 @@ step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict
             const int need = (n + 31) >> 5;
             if (need < live) {
                live = need;
-               LaneWords W;
+               constexpr bool kHeld = TT == kParker && holds_uniform_step<BG, DK, R>();
+               LaneWords<count_members<Lane<R, A>>() + (kHeld ? count_members<UniformStep<R>>() : 0) + 3> W;
                W.n = 0;
                auto put = [&](auto& v) { W.put(v); };
                each_member(L, put);
-               if constexpr (TT == kParker && holds_uniform_step<BG, DK, R>()) each_member(held, put);
+               if constexpr (kHeld) each_member(held, put);
                int flag = fresh;
                put(g); put(attempt); put(flag);
                active = repack_lanes(W, s0, bv, cfg.bnd_slots, active, s_buf);
                W.n = 0;
                auto get = [&](auto& v) { W.get(v); };
                each_member(L, get);
-               if constexpr (TT == kParker && holds_uniform_step<BG, DK, R>()) each_member(held, get);
+               if constexpr (kHeld) each_member(held, get);
                get(g); get(attempt); get(flag);
                fresh = flag != 0;
             }
