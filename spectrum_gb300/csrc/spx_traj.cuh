@@ -846,7 +846,7 @@ template <class R>
 struct UniformStep {
    bool valid;
    V3<R> slope, fa[3];
-   R slope_p, sperp, spara, dtp, dmax, Bmag, divU;
+   R slope_p, sperp, spara, dtp, Bmag, divU;
    StepLimits<R> lim;
 };
 
@@ -890,7 +890,6 @@ __device__ __noinline__ void uniform_step(const ProblemDescT<R>& P, int deriv_mo
    h.fa[2] = sp.bhat;
    h.fa[0] = second_unit(sp.bhat);
    h.fa[1] = cross(h.fa[2], h.fa[0]);
-   h.dmax = sp.dmax;
    const DmaxLimits<R> lim{sp.dmax};
    h.lim = {lim.none(), lim.least(), lim.error()};
    h.Bmag = sp.Bmag;
@@ -1985,7 +1984,7 @@ __device__ __forceinline__ constexpr void each_member(UniformStep<R>& h, F f)
    h.valid = valid != 0;
    f(h.slope.x); f(h.slope.y); f(h.slope.z);
    for (int k = 0; k < 3; k++) { f(h.fa[k].x); f(h.fa[k].y); f(h.fa[k].z); }
-   f(h.slope_p); f(h.sperp); f(h.spara); f(h.dtp); f(h.dmax); f(h.Bmag); f(h.divU);
+   f(h.slope_p); f(h.sperp); f(h.spara); f(h.dtp); f(h.Bmag); f(h.divU);
    f(h.lim.none_); f(h.lim.least_); f(h.lim.error_);
 }
 template <class T>
