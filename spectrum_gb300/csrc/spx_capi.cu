@@ -476,12 +476,13 @@ void set_rk(const spx_ctx* c, spx::RunConfig& cfg)
          if (p.pd.d[d].kind == spx::kDsLossCone) cfg.track_bmag = 1;
 }
 
-// Trajectories per lane of the deep build (58,368 lanes on a GB300) up to which an untuned FP32 run takes it.
-// Measured, wide against deep build: in a uniform field trajectories take the same steps and a launch has no
-// drain to speak of (3e4 trajectories 1.52 / 1.08 ms, 6e4 1.59 / 2.09, 1e6 15.3 / 18.2): one per lane. Lorentz
-// orbits in the dipole (4e5 42.0 / 38.5 ms, 1e6 72.5 / 75.0): ten. Parker trajectories elsewhere differ in
-// length by a factor of ten and more, and the drain lasts as long as the longest (modulation, 1.9e5: 205 /
-// 143 ms, 1.28e6: 411 / 371; shock, 8e5: 151 / 148; grid, 6.4e5: 250 / 206): twenty.
+// Trajectories per lane of the deep build (58,368 lanes on a GB300) up to which an FP32 run takes it.
+// Measured, wide and deep build: in a uniform field trajectories take the same steps and a launch has no
+// drain to speak of (3e4 trajectories 1.08 and 0.68 ms, 5.8e4 1.20 and 0.72, where one each has the lanes full; twice
+// as many take deep lanes twice as long): one per lane. Lorentz orbits in the dipole (4e5 42.0 and 37.8 ms, 5.7e5 50.5
+// and 48.0, 1e6 72.5 and 75.0): ten. Parker trajectories elsewhere differ in length by a factor of ten and more, and
+// the drain lasts as long as the longest (modulation, 1.9e5: 213 and 145 ms, 1.15e6: 394 and 349; shock, 8e5: 102
+// and 96; grid, 6.4e5: 256 and 203): twenty.
 int64_t deep_lanes_limit(const spx_ctx* c)
 {
    return c->traj == SPX_TRAJ_LORENTZ ? 10 : (c->bg_kind == spx::kBgUniform ? 1 : 20);

@@ -67,9 +67,9 @@ template <> struct Lim<float> {
 // correctly rounded and q within an ulp of the quotient, q' is the IEEE quotient bit for bit. (Checked
 // on 5.7e9 of the hardest pairs, which lie next to the middle of two doubles: all equal, no q an ulp away.) Outside the
 // exponent range where no step can over- or underflow (infinities and NaN included) the division itself runs; a zero
-// keeps its sign. In float a quotient is the plain (approximate) division. Measured on one GB300 when it
-// came (FP64): guiding centres in the dipole 521 -> 331 ms, Lorentz orbits 81 -> 68 ms, modulation with numerical
-// derivatives 960 -> 855 ms.
+// keeps its sign. In float a quotient is the plain (approximate) division. One GB300, with the division and with this
+// (FP64, small launches): guiding centres in the dipole 226 and 184 ms, modulation with numerical
+// derivatives 246 and 214 ms, Lorentz orbits 54.8 and 53.3 ms.
 static __device__ __noinline__ double quot_ieee(double x, double y) { return x / y; }
 
 template <class R> struct Divisor;

@@ -49,17 +49,18 @@ enum BndKind : int {
 // passing) and no momentum boundary, the set-up of the heliospheric modulation runs. kLayoutPlanes: one such
 // time boundary, two planes and one momentum boundary (injection or pass), the set-up of diffusive shock
 // acceleration. kLayoutTime: one such time boundary and no other, pure diffusion.
-// (On one GB300 the shock's launch of 4e4 trajectories went from 455 to 277 ms with its layout and the one-bit kind
-// tests of eval_space_bnd: a boundary's dependent loads and branches cost a lone warp more than its arithmetic. Pure
-// diffusion of 1e6: 15.3 to 11.3 ms.)
+// (One GB300, kernels of the diffusion class without and with the layout: shock acceleration of 4e4 trajectories 375 and
+// 251 ms, a boundary's dependent loads and branches cost a lone warp more than its arithmetic; pure diffusion of 1e6
+// 15.0 and 11.3 ms.)
 enum BndLayout : int { kLayoutAny = 0, kLayoutSpheres = 1, kLayoutPlanes = 2, kLayoutTime = 3 };
 
 // Resident blocks of 128 threads per SM the register allocation is sized for. The FP32 kernels come in two
 // builds. Wide, five blocks (20 warps, at most 102 registers), has the most steps per second with every lane
 // busy: the extra warps hide more dependent-instruction latency than the spilled values cost (four blocks ran
 // 2-5% slower). Deep, three blocks, spills nothing, so a warp's step is shorter: it is the faster one where a
-// launch is mostly its drain, the last trajectories alone on the SMs. One GB300, wide to deep with its repacking: shock acceleration of 4e4
-// trajectories 580 -> 453 ms, modulation of 1.9e5 325 -> 245 ms, on a 256^3 grid 530 -> 375 ms.
+// launch is mostly its drain, the last trajectories alone on the SMs. One GB300, wide and deep (with its repacking): shock
+// acceleration of 4e4 trajectories 402 and 251 ms, modulation of 1.9e5 333 and 245 ms, on a 256^3 grid 505 and 337 ms,
+// 2e5 Lorentz orbits 32.1 and 26.6 ms.
 constexpr int kWideBlocksF32 = 5, kDeepBlocksF32 = 3, kBlocksF64 = 1;
 
 enum IniKind : int {

@@ -531,8 +531,8 @@ __device__ __forceinline__ bool grid_fields(const BgParamsT<R>& g, V3<R> pos, un
 // memory hold the team size, a power of two; the lanes of a team are neighbours and run the same trajectory
 // with the same numbers. They share out the points of finite differences and the halves of a Box-Muller
 // block: the FP64 pipe takes as long for one lane as for 32, so a launch too small to fill the lanes has
-// them for nothing. One GB300: 1,200 modulation trajectories with numerical
-// derivatives 855 -> 307 ms in teams of eight, 254 ms with the rows of the gradients shared out as well.
+// them for nothing. One GB300: 1,200 modulation trajectories with numerical derivatives take 512 ms with one lane each
+// in full warps, 214 ms in teams of eight over all schedulers.
 extern __shared__ __align__(16) unsigned char spx_smem[];
 struct Team {
    int size, rank;
@@ -1071,8 +1071,9 @@ __device__ __forceinline__ void eval_space_bnd(const BndParamsT<R>& b, BndState<
 // The distance that a point at "delta" from the boundary can move without crossing it: |delta| of a sphere or
 // plane less what rounding may add to it, with the coordinates' sum of magnitudes as "reach"; 0 (not known) for the
 // other kinds. The stage points of a Runge-Kutta step, a small part of the way to the nearest boundary, are told by
-// it with one comparison instead of an evaluation of every boundary. One GB300: focused transport with three
-// spheres 425 -> 326 ms, Lorentz orbits 36.7 -> 33.5 ms.
+// it with one comparison instead of an evaluation of every boundary, and the steps' ends as long as it lasts
+// (handle_boundaries). One GB300, without and with both: focused transport with three spheres 418 and 283 ms,
+// Lorentz orbits 31.4 and 26.6 ms, shock acceleration 262 and 251 ms; modulation the same.
 template <int BL, class R>
 __device__ __forceinline__ R bnd_clearance(const BndParamsT<R>& b, R delta, R reach)
 {

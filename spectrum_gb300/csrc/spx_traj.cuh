@@ -3,12 +3,16 @@
 // Euler pitch-angle scattering step), boundary handling, distribution events, and the kernel
 // that schedules trajectories onto lanes.
 //
-// One lane integrates one trajectory. The state a lane carries from step to step is only time,
-// position, momentum, weights, the time-step memory and the boundary deltas; the fields are
+// One lane integrates one trajectory, in small FP64 launches a team of up to eight lanes (Team), all with the same
+// numbers. The state a lane carries from step to step is time, position, momentum, weights, the time-step memory, the
+// boundary deltas and how far it may go before the spatial boundaries are evaluated again; in a uniform field
+// also the coefficients that do not change along a trajectory (UniformStep). Elsewhere the fields are
 // evaluated at the start of every step (the reference evaluates them at the end of the previous
-// step, src/trajectory_parker.cc:300, which gives the same values). The plain schedule gives
-// lane k the trajectories k, k + stride, ...; the queue schedule refills finished lanes from a
-// global work-queue counter, one atomic per warp and refill, lanes ranked with __ballot_sync/__popc.
+// step, src/trajectory_parker.cc:300, which gives the same values). The plain schedule gives the
+// RunConfig::warp_lanes lanes at work in each warp, in teams, the trajectories k, k + stride, ...; the queue schedule
+// refills finished lanes from a global work-queue counter, one atomic per warp and refill, lanes ranked with
+// __ballot_sync/__popc. When no trajectories are left to start, the blocks of most kernels move the states of the
+// lanes still at work into as few warps as hold them (repack_lanes).
 #pragma once
 
 #include "spx_physics.cuh"
@@ -265,8 +269,8 @@ static __device__ __noinline__ V3<double> sample_mom(InitRng& rng, const Problem
 // The event's "second point" is the current state; its spatial data are the fields of the
 // step's start point, as in the reference (HandleBoundaries runs before CommonFields). It is kept as the
 // kernel has it and turned into doubles where an event reads it: in the FP32 kernels every conversion
-// holds the FP64 pipe, and a guiding-centre orbit bins a mirror point every hundred steps (1e5 orbits of ten
-// seconds: 38.4 -> 36.5 ms; an event with no weight also leaves out the exponential).
+// holds the FP64 pipe, and a guiding-centre orbit bins a mirror point every hundred steps (when it came, 1e5 orbits
+// of ten seconds took 36.5 ms instead of 38.4; an event with no weight also leaves out the exponential).
 template <class R, class A>
 struct EventPoint {
    A t_;
@@ -556,9 +560,9 @@ __device__ __forceinline__ int n_mom_bnd(const ProblemDescT<R>& P) { return BL =
 // boundary can have been crossed, and none is evaluated (a state's delta_old is then an older one of the same sign;
 // of an absorbing or passing boundary only the sign is read). In double it is the difference of the positions: the
 // increments fall short of it by their rounding, which a field that drives every step alike adds up. (The sums of the
-// float kernels lose 2^-48 of the position a step, in 10^7 steps a thousandth of bnd_clearance's margin.) One GB300: focused transport 326 -> 286 ms, shock
-// acceleration 286 -> 268 ms, modulation 245 -> 238 ms. Not in the wide FP32 Parker kernels, whose warps wait for issue
-// slots and registers, not for the evaluation (modulation with every lane busy 4.84e10 -> 4.61e10 steps/s with it).
+// float kernels lose 2^-48 of the position a step, in 10^7 steps a thousandth of bnd_clearance's margin.) What it gives
+// stands at bnd_clearance. Not in the wide FP32 Parker kernels, whose warps wait for issue slots and registers, not for
+// the evaluation (modulation with every lane busy: 4.61e10 steps/s with it, 4.84e10 without).
 template <int TT, int BL, bool CL, class R, class A, class F>
 __device__ __forceinline__ void handle_boundaries(Lane<R, A>& L, BndView<R> bv, const SD<R>& sp, const Start& s0,
                                                   const ProblemDescT<R>& P, const ProblemDesc& Pd, const Sinks& S, F moved)
@@ -840,8 +844,8 @@ __device__ __forceinline__ void step_normals(uint4 b, double n[4])
 // PhysicalStep -- is the same at every point, and div U = 0 keeps the momentum. It is evaluated at the first
 // step of an attempt by the general code and held in registers; a later step draws its normals, moves and
 // tests its boundaries. The same operations on the same numbers: the trajectories do not change.
-// One GB300, 1e5 trajectories of 1,000 steps in FP64: 184.7 -> 44.0 ms (a step was 930 FP64 instructions, six of
-// its seven field evaluations for a divergence that is zero); 1e6 in FP32: 16.5 -> 14.6 ms.
+// One GB300, 1e5 trajectories of 1,000 steps in FP64: 156.5 ms with the general step, 40.5 ms with this (the general one
+// makes seven field evaluations, six of them for a divergence that is zero); 1e6 in FP32 12.9 and 11.3 ms.
 template <class R>
 struct UniformStep {
    bool valid;
@@ -1345,7 +1349,8 @@ struct SplitVector {
 // in the order that one lane adds them. The operations are those of get_fields, vel_cart and rk_slopes
 // (guiding_drift for TrajectoryGuiding), with what vanishes in the dipole left out: E, and curl B, whose
 // differences of equal entries of the symmetric grad B are zero. False on a field error. One
-// GB300: 512 guiding centres 281 -> 201 ms, 4,001 Lorentz orbits 58.0 -> 53.8 ms.
+// GB300, teams without and with it (and the split sums of the steps): 512 guiding centres 276 and 184 ms, 4,001 Lorentz
+// orbits 61.5 and 53.3 ms.
 template <int TT>
 __device__ __noinline__ bool dipole_slopes_split(const BgParams& g, V3<double> pos, V3<double> mom, SD<double>& s, V3<double>& vel,
                                                  V3<double>& sp, V3<double>& sm)
@@ -1678,8 +1683,8 @@ __device__ __forceinline__ void rk_advance(Lane<R, A>& L, BndView<R> bv, Start& 
       }
       else {
          // the fixed tables have one nonzero coefficient a stage, that of the stage before; the reference
-         // advances t once for every earlier stage. (Adding the zero products cost ten float operations each:
-         // the FP32 dipole orbits take 42.4 ms instead of 51.0, guiding centres 38.4 instead of 43.6.)
+         // advances t once for every earlier stage. (Adding the zero products costs ten float operations each:
+         // when they went, the FP32 dipole orbits took 42.4 ms instead of 51.0, guiding centres 38.4 instead of 43.6.)
          const R dta = tab.template a<R>(is) * L.dt, ds = fwd ? dta : -dta;
 #pragma unroll
          for (int il = 0; il < is; il++) acc_add(L.t, ds);
@@ -1852,8 +1857,8 @@ __device__ __noinline__ void set_start(Lane<R, A>& L, BndView<R> bv, Start& s0, 
    V3<R> pr = val3<R>(L.pos);
    // The momentum is sampled twice, first for the momentum that the field evaluation takes (about (1, 1, 1)), then
    // about the field. Only numerical derivatives read the first; elsewhere its draws are skipped, unless the
-   // attempt ends here and leaves it in the record. (Set-up is FP64 work: skipping it took 2e5 FP32 Lorentz orbits in
-   // the dipole from 32.5 to 30.3 ms.)
+   // attempt ends here and leaves it in the record. (Set-up is FP64 work: 2e5 FP32 Lorentz orbits in the
+   // dipole take 27.0 ms with the sample and 26.6 without; 32.5 and 30.3 when every start held its warp.)
    constexpr bool kReadsMom = kFP64 && (BG == kBgSolarWind || BG == kBgGrid);
    const InitRng before = rng;
    V3<double> mom = mk(0.0, 0.0, 0.0);
@@ -1949,8 +1954,10 @@ __device__ __forceinline__ void start_lane(Lane<R, A>& L, BndView<R> bv, Start& 
 // lanes each: as many warps issue as at the start, for a fraction of the steps. When the block's active lanes
 // fit in fewer warps, their states move to the first threads and the warps left empty wait at the block's
 // barrier, so the others have the schedulers (and in FP64 the pipe, which a warp occupies as long for one
-// lane as for 32). A block repacks at most blockDim / 32 - 1 times. Without it the deep build
-// took 499, 270 and 405 ms on the three runs given below, with it 453, 245 and 375.
+// lane as for 32). A block repacks at most blockDim / 32 - 1 times. One GB300, FP32 without and
+// with it: shock acceleration of 4e4 trajectories 291 and 251 ms, modulation of 1.9e5 264 and 245 ms, on a 256^3 grid
+// 362 and 337 ms, 1e5 guiding centres 31.5 and 26.6 ms (2e5 47.5 and 42.9, 1e3 the same; focused transport lost 4%
+// below 1e5 trajectories, and has no build that repacks).
 
 // Lane state as words, for the exchange below: room for N of them.
 template <int N>
@@ -2032,18 +2039,6 @@ __device__ __noinline__ bool repack_lanes(LaneWords<N>& W, Start& s0, BndView<R>
    return mine;
 }
 
-// One lane per thread. Dynamic shared memory holds the lanes' boundary states
-// (boundaries per lane x blockDim.x x sizeof(BndState<R>)).
-// DM is the field-derivative method (SPX_OPT_DERIV_MODE) fixed per instantiation, so the analytic
-// kernels carry no finite-difference code (whose out-of-line calls would pin the field record to
-// the stack).
-// DK >= 0: a kernel specialised for one diffusion class (the Parker types); -1 dispatches at run time;
-// kDkNoDiffusion: the guiding-centre kernels for TrajectoryGuiding proper (no scattering, no perpendicular step).
-// BL: the boundary layout (BndLayout) the Parker step is compiled for; kLayoutAny reads it from the
-// descriptor.
-// MB: resident blocks of 128 per SM (above); the wide FP32 build does not repack its lanes, but for the guiding
-// centres, which have no other: orbits' step counts differ by a factor of five, and repacking took 1e5 of them from
-// 32.3 to 26.6 ms (2e5 27.2 -> 25.0, 1e3 7.56 -> 7.29; focused transport lost 4% below 1e5 trajectories).
 // Steps between two barriers of a draining block: few enough that a warp emptied early is soon given up,
 // enough that waiting for the slowest of the block's warps costs little (32 to 128 are within 2% of each other;
 // grid transport 366 ms at 32, 355 at 64).
@@ -2052,11 +2047,22 @@ constexpr int kDrainSteps = 64;
 // The FP32 Lorentz kernels start trajectories several at a time. A start is FP64 work that holds its warp as long for
 // one lane as for all of them, and at a thousand steps an orbit a lane of the warp ends every thirty: starts took a
 // quarter of the time. A lane waits until kRefillLanes of its warp are idle, about kWaitSteps steps at the most, so that
-// orbits far longer than that lose nothing. Dipole, 2e5 orbits 30.2 -> 25.9 ms, 4e5 50.0 -> 42.0, 1e6 94.9 -> 72.5
-// (128 steps: 26.3, 42.9, 75.2). Guiding centres gained 5% at 5e5 and lost 5% below
+// orbits far longer than that lose nothing. Dipole, without and with it: 2e5 orbits 30.7 and 26.6 ms, 4e5 48.1 and
+// 37.8, 1e6 95.3 and 73.5 (a wait of 128 steps was 2-4% slower). Guiding centres gained 5% at 5e5 and lost 5% below
 // 1e5; Parker and focused trajectories are longer, and start too rarely for it to show.
 constexpr int kRefillLanes = 16;
 
+// One lane per thread. Dynamic shared memory holds a header and the lanes' boundary states
+// (boundaries per lane x blockDim.x x sizeof(BndState<R>)).
+// DM is the field-derivative method (SPX_OPT_DERIV_MODE) fixed per instantiation, so the analytic
+// kernels carry no finite-difference code (whose out-of-line calls would pin the field record to
+// the stack).
+// DK >= 0: a kernel specialised for one diffusion class (the Parker types); -1 dispatches at run time;
+// kDkNoDiffusion: the guiding-centre kernels for TrajectoryGuiding proper (no scattering, no perpendicular step).
+// BL: the boundary layout (BndLayout) the Parker step is compiled for; kLayoutAny reads it from the
+// descriptor.
+// MB: resident blocks of 128 per SM. The wide FP32 build does not repack its lanes, but for the guiding
+// centres, which have no other and whose orbits' step counts differ by a factor of five.
 template <int TT, int BG, class R, int DM, bool GT, int DK, int BL, int MB>
 __global__ void __launch_bounds__(128, MB)
 step_kernel(const ProblemDescT<R>* __restrict__ P, const ProblemDesc* __restrict__ Pd, RunConfig cfg,
