@@ -494,7 +494,8 @@ __device__ __forceinline__ void handle_crossings(Lane<R, A>& L, BndView<R> bv, c
       const BndParamsT<R>& b = P.bs[i];
       BndState<R> st = bv.ld(j);
       if (b.reflect) {
-         // src/trajectory_base.cc:462-483: mirror the position, reverse the momentum
+         // src/trajectory_base.cc:462-483: mirror the position, reverse the momentum; distance and normal are those of
+         // the point where the step's boundaries were evaluated, also after an earlier one of them has mirrored it
          V3<R> shift = (R(2) * st.delta) * bnd_normal(b, pos);
          add3(L.pos, R(-1) * shift);
          // ReverseMomentum: the base negates the vector (src/trajectory_base.cc:139-142; Lorentz and
@@ -503,9 +504,7 @@ __device__ __forceinline__ void handle_crossings(Lane<R, A>& L, BndView<R> bv, c
          if (TT == kLorentz || TT == kFieldline) { L.mom.x = neg(L.mom.x); L.mom.y = neg(L.mom.y); L.mom.z = neg(L.mom.z); }
          else if (TT == kFocused) L.mom.y = neg(L.mom.y);
          else if (TT == kGuiding) L.mom.z = neg(L.mom.z);
-         pos = val3<R>(L.pos);
-         mom = lane_mom(L);
-         compute_bnd<1>(b, st, L.t, pos, mom, sp.bhat, sp.region, TT);
+         compute_bnd<1>(b, st, L.t, val3<R>(L.pos), lane_mom(L), sp.bhat, sp.region, TT);
          st.crossings_left--;
          bv.st(j, st);
       }
@@ -521,6 +520,8 @@ __device__ __forceinline__ void handle_crossings(Lane<R, A>& L, BndView<R> bv, c
    }
    if (active >= 0) distro_events<TT>(L, sp, s0, Pd, active, S);
    // RecordBoundary of the crossed ones, in slot order
+   pos = val3<R>(L.pos);
+   mom = lane_mom(L);
    for (int j = 0; j < s_lo; j++)
       if (crossed & (1u << j)) {
          BndState<R> st = bv.ld(j);

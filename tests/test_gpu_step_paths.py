@@ -8,6 +8,7 @@
 - The deep build of the FP32 kernels, with its repacking of lanes, against the wide one.
 - The initial momentum, of whose two samples the first is only counted where nothing reads it, against the oracle.
 - Small FP64 launches: teams of lanes sharing a trajectory against one lane each.
+- Steps that cross two reflecting boundaries, against the oracle.
 - Launches of few trajectories keep their shape when the autotuner has run or when a run is given back what another
   reported; larger ones take the tuned shape.
 - Uniform fields: coefficients held over a trajectory (diffusion classes that do not read the position)
@@ -306,3 +307,19 @@ def test_larger_launches_take_the_tuned_shape(built_lib, precision, n):
         assert _shape(sim.MainLoop().tuning) == _shape(best) and best.blocks_per_sm > 0
     finally:
         sim.close()
+
+
+@pytest.mark.parametrize("kind", ["sphere_plane", "plane_sphere", "two_spheres", "box_sphere"])
+def test_two_reflections_in_one_step_match_oracle(built_lib, kind):
+    """Long steps that cross two reflecting boundaries at once: each mirrors with its distance and normal at the step's
+    end, where the first has not moved the point yet."""
+    c = cases
+    sphere = (c.BoundarySphereReflect(), c.B(DC(), -1, [-1]).vec((0, 0, 0)).double(0.4))
+    plane = (BoundaryPlaneReflect(), c.B(DC(), -1, [-1]).vec((0.15, 0, 0)).vec((1.0, 0.5, 0)))
+    bnds = {"sphere_plane": [sphere, plane], "plane_sphere": [plane, sphere],
+            "two_spheres": [sphere, (c.BoundarySphereReflect(), c.B(DC(), -1, [-1]).vec((0.2, 0, 0)).double(0.4))],
+            "box_sphere": [c.BOUNDARY_CASES["box_reflect"], sphere]}[kind]
+    bg = (c.BackgroundUniform(), DC().double(0.0).vec((0, 0, 0)).vec((0, 0, 0)).vec((0, 0.3, 1.0)).double(0.2))
+    pb = c._parker(n=400, bg=bg, t_end=0.2, bnds=bnds, is_=(c.InitialSpaceFixed(), DC().vec((0.05, 0, 0))))
+    res = run_problems(pb, precision=capi.SPX_FP64, record=True)
+    ot.assert_fp64_parity(res.records[0], ot.run_oracle(pb), ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
