@@ -1084,6 +1084,10 @@ __device__ __forceinline__ R bnd_clearance(const BndParamsT<R>& b, R delta, R re
    return m_max(m_abs(delta) - eps * (reach + norm1(ld3(b.origin)) + b.radius), R(0));
 }
 
+// |mom| as a call: few guiding-centre runs have a momentum boundary, and its code inlined beside the mirror points' took
+// the FP64 orbits in the dipole from 183.5 to 186.1 ms.
+template <class R> __device__ __noinline__ R norm_call(V3<R> a) { return norm(a); }
+
 template <int BL, class R>
 __device__ __forceinline__ void eval_mom_bnd(const BndParamsT<R>& b, BndState<R>& st, V3<R> pos, V3<R> mom,
                                              V3<R> bhat, int traj)
@@ -1098,7 +1102,9 @@ __device__ __forceinline__ void eval_mom_bnd(const BndParamsT<R>& b, BndState<R>
       st.delta = (traj == kFocused) ? mom.x * mom.y : (traj == kGuiding ? mom.z : dot(mom, bhat));
       return;
    }
-   st.delta = (traj == kLorentz ? norm(mom) : mom.x) - b.momentum;
+   // the magnitude, which Lorentz and the guiding-centre types form from components (src/boundary_momentum.cc:69-75)
+   if (traj == kGuiding) st.delta = norm_call(mom) - b.momentum;
+   else st.delta = (traj == kLorentz ? norm(mom) : mom.x) - b.momentum;
    if (b.kind == kBtMomentumSlab && st.delta * st.delta_old < R(0)) {
       if (dot(pos - ld3(b.slab_r0), ld3(b.slab_n)) * dot(pos - ld3(b.slab_r1), ld3(b.slab_n)) > R(0)) st.delta_old = st.delta;
    }

@@ -191,3 +191,20 @@ def test_perpendicular_spread(built_lib, precision):
     assert abs(r2.mean() - expect) < 4.0 * sigma, (r2.mean(), expect, sigma)
     np.testing.assert_allclose(np.linalg.norm(rec["mom"], axis=1), np.linalg.norm(rec["mom0"], axis=1), rtol=1e-4)
 
+
+@pytest.mark.parametrize("kind,fraction", [("pass", 0.9), ("inject", 0.9), ("pass", 1.0 - 1.0e-6)])
+def test_momentum_boundary_takes_the_magnitude(built_lib, kind, fraction):
+    """A momentum boundary of guiding centres, whose components change along every bounce, lies at a magnitude of the
+    momentum: the orbits keep it to 1e-6, so at 0.9 of it nothing crosses, and a few orbits do just below it."""
+    from spectrum_gb300.datacontainer import DataContainer as DC
+    from spectrum_gb300.plugins import BoundaryMomentumInject, BoundaryMomentumPass
+    cls, crossings = (BoundaryMomentumPass, -1) if kind == "pass" else (BoundaryMomentumInject, 1)
+    pb = make_golden._guiding_dipole(64)
+    pb.AddBoundary(cls(), workloads._boundary(DC(), crossings, [-1, 0]).double(fraction * U.mev_to_mom(10.0)))
+    res, ref = run_problems(pb, precision=capi.SPX_FP64, record=True), ot.run_oracle(pb)
+    ot.assert_fp64_parity(res.records[0], ref, ot.run_oracle(pb, nudge_libm=1), distros=res.distros[0])
+    mirrors = ot.run_oracle(make_golden._guiding_dipole(64)).distros[1][2]
+    assert ref.distros[1][2] == mirrors if fraction < 0.99 else ref.distros[1][2] > mirrors
+    if fraction < 0.99:
+        rec = run_problems(pb, precision=capi.SPX_MIXED, record=True).records[0]
+        assert not np.any(rec["status"] & 0x0080)  # the bit of a momentum boundary
